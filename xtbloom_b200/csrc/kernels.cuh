@@ -162,6 +162,10 @@ void launch_tridiag_smem(const EigArgs& g, const int32_t* list, int count, int m
 // Register-resident cluster tridiagonalisation for systems with n <= tridiag_reg_max_n().
 int tridiag_reg_max_n();
 void launch_tridiag_reg(const EigArgs& g, const int32_t* list, int count, int max_n, cudaStream_t stream);
+// Cluster tridiagonalisation with the matrix in global memory, for systems
+// above the register-resident kernel's size.
+bool tridiag_large_fits(int max_n);
+void launch_tridiag_large(const EigArgs& g, const int32_t* list, int count, int max_n, cudaStream_t stream);
 size_t tridiag_smem_bytes(int nl, int nt);
 int sm_count();   // multiprocessors of the current device (cached)
 // max_levels: the most eigenvalues a system of the launch needs in the SCC
