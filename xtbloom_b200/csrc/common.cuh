@@ -169,6 +169,14 @@ __device__ __forceinline__ double logistic(double x) {
   return e / (1.0 + e);
 }
 
+// One FP64 tensor-core product D = A B + D of an 8x8x4 tile (warp-wide):
+// lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4) .. 2(l%4)+1].
+__device__ __forceinline__ void mma_f64(double* d, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

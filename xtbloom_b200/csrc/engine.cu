@@ -1439,22 +1439,10 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
       launch_inverse_iteration(sub(bk), bk.count, bk.max_n,
                                mode != 0 ? bk.max_n : std::min(bk.max_m + 4, bk.max_n), ortol_rel, st);
     };
-    auto wy_cap = [&](const Bucket& bk) {
+    // the T factors (launch_wy_factor) are formed before
+    auto backtransform = [&](const Bucket& bk, cudaStream_t st) {
       const int want = mode != 0 ? bk.max_n : std::min(bk.max_m, bk.max_n);
-      const long budget = 220L * 1024 / 8 - (long)bk.max_n * 33 - 32 * 33 - 8;
-      return (int)std::min<long>(want, budget / 32);
-    };
-    // factored: the T factors were launched already (launch_wy_factor)
-    auto backtransform = [&](const Bucket& bk, cudaStream_t st, bool factored = false) {
-      const EigArgs gb = sub(bk);
-      const int want = mode != 0 ? bk.max_n : std::min(bk.max_m, bk.max_n);
-      const int wcap = wy_cap(bk);
-      if (wcap >= 8) {
-        launch_backtransform_wy(gb, bk.count, bk.max_n, wcap, want, st, factored);
-      } else {
-        // a block of reflectors no longer fits in shared memory: row chunks
-        launch_backtransform_rows(gb, bk.count, bk.max_n, want, st);
-      }
+      launch_backtransform(sub(bk), bk.count, bk.max_n, want, st);
     };
     if (!bks.empty() && !m.prof.on && m.ensure_bucket_streams()) {
       // Each bucket runs its whole chain on its own side stream, forked from
@@ -1469,17 +1457,14 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
         const int k = (int)(i % Impl::kBucketStreams);
         cudaStream_t st = m.bst[k];
         tridiag(bks[i], st);
-        const bool fork = wy_cap(bks[i]) >= 8;
-        if (fork) {
-          cudaEventRecord(m.ffork[k], st);
-          cudaStreamWaitEvent(m.fst[k], m.ffork[k], 0);
-          launch_wy_factor(sub(bks[i]), bks[i].count, bks[i].max_n, m.fst[k]);
-          cudaEventRecord(m.wydone[k], m.fst[k]);
-        }
+        cudaEventRecord(m.ffork[k], st);
+        cudaStreamWaitEvent(m.fst[k], m.ffork[k], 0);
+        launch_wy_factor(sub(bks[i]), bks[i].count, bks[i].max_n, m.fst[k]);
+        cudaEventRecord(m.wydone[k], m.fst[k]);
         eigvals(bks[i], st);
         invit(bks[i], st);
-        if (fork) cudaStreamWaitEvent(st, m.wydone[k], 0);
-        backtransform(bks[i], st, fork);
+        cudaStreamWaitEvent(st, m.wydone[k], 0);
+        backtransform(bks[i], st);
       }
       for (int i = 0; i < ns; ++i) {
         cudaEventRecord(m.bjoin[i], m.bst[i]);
@@ -1496,7 +1481,10 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
     XTB_STAGE(stage_base == kStLowdin ? kStLowdin : kStInvIter, (int)bks.size(),
               for (const Bucket& bk : bks) invit(bk, s));
     XTB_STAGE(stage_base == kStLowdin ? kStLowdin : kStBacktransform, (int)bks.size(),
-              for (const Bucket& bk : bks) backtransform(bk, s));
+              for (const Bucket& bk : bks) {
+                launch_wy_factor(sub(bk), bk.count, bk.max_n, s);
+                backtransform(bk, s);
+              });
   };
 
   // ---- Loewdin orthogonaliser X = U s^-1/2 U^T ----

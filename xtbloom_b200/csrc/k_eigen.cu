@@ -28,14 +28,6 @@ namespace xtb {
 
 constexpr int GB = 64, GK = 16;
 
-// One FP64 tensor-core product D = A B + D of an 8x8x4 tile (warp-wide):
-// lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4) .. 2(l%4)+1].
-__device__ __forceinline__ void mma_f64(double* d, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 // FP64 tile (ti, tj) of edge TB (64, or 32 when few systems are active) of
 // system s on the FP64 tensor cores (mma.m8n8k4.f64, FP64 accumulation):
 // 256 threads as 2 x 4 warps, each warp a (TB/2) x (TB/4) block of 8x8
@@ -1300,10 +1292,9 @@ __global__ void __launch_bounds__(kInvSmemThreads) k_inverse_iteration_smem(EigA
 
 
 // ---------------------------------------------------------------------------
-// Blocked back-transform (compact WY form, LAPACK larft/larfb order): the
+// Compact-WY factors of the back-transform (k_backtransform.cu): the
 // reflectors H_i0 ... H_i0+31 of one block are I - V T V^T with T upper
-// triangular, so each block costs one pass over Z: Z <- Z - V (T (V^T Z)).
-// Blocks are applied from the last to the first.
+// triangular.
 // ---------------------------------------------------------------------------
 constexpr int WB = 32;
 
@@ -1357,10 +1348,6 @@ __device__ __forceinline__ void load_wy_block(const double* a, int n, int i0, in
 }
 
 size_t wy_factor_bytes(int n) { return ((size_t)n * (WB + 1) + 2 * WB * (WB + 1)) * sizeof(double); }
-
-size_t backtransform_wy_bytes(int n, int m) {
-  return ((size_t)n * (WB + 1) + WB * (WB + 1) + (size_t)WB * m + 8) * sizeof(double);
-}
 
 // T factor of every 32-reflector block (LAPACK larft, forward columnwise):
 // H_i0 ... H_i0+k-1 = I - V T V^T with T upper triangular,
@@ -1416,299 +1403,10 @@ __global__ void __launch_bounds__(256) k_wy_factor(EigArgs g) {
   }
 }
 
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// load_wy_block and the T factor of block b, issued as asynchronous copies
-// (one commit group) so that they overlap the work on the previous block;
-// the unit diagonal and the zeros above it are plain stores.
-__device__ __forceinline__ void prefetch_wy_block(const double* a, const double* tf, int n, int nr,
-                                                  int b, double* V, double* T) {
-  constexpr int P = WB + 1;
-  const int i0 = b * WB, k = min(WB, nr - i0), L = n - i0 - 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int c = warp; c < WB; c += nw) {
-    const double* row = a + (int64_t)(i0 + c) * n + i0 + 1;
-    for (int r = lane; r < L; r += 32) {
-      double* dst = V + r * P + c;
-      if (c < k && r > c) cp_async8(dst, row + r);
-      else *dst = (c < k && r == c) ? 1.0 : 0.0;
-    }
-  }
-  for (int idx = threadIdx.x; idx < WB * WB; idx += blockDim.x)
-    cp_async8(T + (idx / WB) * P + (idx % WB), tf + (int64_t)b * WB * WB + idx);
-  cp_async_commit();
-}
-
-// Blocked back-transform (compact WY form, LAPACK larfb order): each block of
-// 32 reflectors costs one pass over Z: Z <- Z - V (T (V^T Z)), blocks from the
-// last to the first, T from k_wy_factor.  Grid (parts, systems): part
-// blockIdx.x transforms its contiguous slice of the system's eigenvectors
-// (parts > 1 only when few systems are active, so that one system's vectors
-// are spread over several SMs).  STAGED: the slice lives in shared memory for
-// the whole pass (few vectors per CTA), so no block waits on global loads of Z.
-template <bool STAGED>
-__global__ void __launch_bounds__(256) k_backtransform_wy(EigArgs g, int wcap, int per_cap) {
-  extern __shared__ double sm[];
-  const int s = g.list[blockIdx.y];
-  if (g.only != nullptr && g.only[s] == 0) return;
-  const int n = g.nao[s];
-  const int mt = g.all_vectors ? n : g.nvec[s];
-  const int per = (mt + gridDim.x - 1) / gridDim.x;
-  const int jbeg = blockIdx.x * per;
-  const int m = min(mt - jbeg, per);
-  const double* a = g.A + g.mat_off[s];
-  const double* tf = g.scratch + g.scratch_off[s] + wy_t_offset(n);
-  double* gZ = g.Z + g.mat_off[s] + (int64_t)jbeg * n;
-  const int nr = n - 2;
-  if (nr <= 0 || m <= 0) return;
-  const int tid = threadIdx.x, bs = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = bs >> 5;
-  constexpr int P = WB + 1;
-  // V (n x P) and T (WB x P) of one block; STAGED keeps two of each so that
-  // the next block arrives by cp.async while this one is applied
-  double* V0 = sm;
-  double* T0 = V0 + (size_t)n * P;
-  double* V1 = STAGED ? T0 + WB * P : V0;
-  double* T1 = STAGED ? V1 + (size_t)n * P : T0;
-  double* W = T1 + WB * P;               // WB x wcap
-  // per_cap x n staging buffer; a slice larger than planned stays in global memory
-  const bool stage = STAGED && per <= per_cap;
-  double* Z = stage ? W + (size_t)WB * wcap : gZ;
-  if (stage)
-    for (int64_t k = tid; k < (int64_t)m * n; k += bs) Z[k] = gZ[k];
-  const int nblk = (nr + WB - 1) / WB;
-  if (STAGED) prefetch_wy_block(a, tf, n, nr, nblk - 1, V0, T0);
-  for (int it = 0; it < nblk; ++it) {
-    const int b = nblk - 1 - it;
-    const int i0 = b * WB;
-    const int k = min(WB, nr - i0);
-    const int L = n - i0 - 1;
-    const bool odd = STAGED && (it & 1);
-    double* V = odd ? V1 : V0;
-    double* T = odd ? T1 : T0;
-    if (STAGED) {
-      if (b > 0) {
-        prefetch_wy_block(a, tf, n, nr, b - 1, odd ? V0 : V1, odd ? T0 : T1);
-        cp_async_wait<1>();   // this block's copies are done, the next one's may fly
-      } else {
-        cp_async_wait<0>();
-      }
-    } else {
-      load_wy_block(a, n, i0, k, L, V);
-      for (int idx = tid; idx < WB * WB; idx += bs) {
-        const int p = idx / WB, q = idx - (idx / WB) * WB;
-        T[p * P + q] = tf[(int64_t)b * WB * WB + idx];
-      }
-    }
-    __syncthreads();
-    // eigenvectors in chunks of at most wcap (the W buffer's capacity)
-    for (int j0 = 0; j0 < m; j0 += wcap) {
-    const int jc = min(wcap, m - j0);
-    // W = T (V^T Z_block): one warp per eigenvector, lane = reflector
-    for (int jj = warp; jj < jc; jj += nw) {
-      const int j = j0 + jj;
-      const double* z = Z + (int64_t)j * n + i0 + 1;
-      double acc = 0.0;
-      for (int r0 = 0; r0 < L; r0 += 32) {
-        const double zv = (r0 + lane < L) ? z[r0 + lane] : 0.0;
-        const int rmax = min(32, L - r0);
-        for (int rr = 0; rr < rmax; ++rr) {
-          const double zr = __shfl_sync(0xffffffffu, zv, rr);
-          const int r = r0 + rr;
-          if (lane < k && r >= lane) acc = fma(V[r * P + lane], zr, acc);
-        }
-      }
-      double w2 = 0.0;
-      for (int q = 0; q < WB; ++q) {
-        const double w1 = __shfl_sync(0xffffffffu, acc, q);
-        if (q >= lane) w2 = fma(T[lane * P + q], w1, w2);
-      }
-      W[lane * wcap + jj] = w2;
-    }
-    __syncthreads();
-    for (int64_t idx = tid; idx < (int64_t)jc * L; idx += bs) {
-      const int jj = (int)(idx / L), r = (int)(idx - (idx / L) * L);
-      const int amax = min(k, r + 1);
-      double acc = 0.0;
-      for (int q = 0; q < amax; ++q) acc = fma(V[r * P + q], W[q * wcap + jj], acc);
-      Z[(int64_t)(j0 + jj) * n + i0 + 1 + r] -= acc;
-    }
-    __syncthreads();
-    }
-  }
-  if (stage)
-    for (int64_t k = tid; k < (int64_t)m * n; k += bs) gZ[k] = Z[k];
-}
-
-// Blocked back-transform on the FP64 tensor cores (many systems, one CTA per
-// system): per 32-reflector block, Y = V^T Z (32 x m) as 8 x 8 x 4 DMMA tiles,
-// each warp a strip of four 8-row blocks for one block of eight eigenvectors
-// (one global load of Z feeds four products), W = T Y in shared memory, and
-// Z <- Z - V W as transposed tiles (eigenvector x row: each lane updates two
-// adjacent rows of one eigenvector).  Z stays in global memory (vector-major
-// rows of n), V and T of the block in shared memory.
-__global__ void __launch_bounds__(256) k_backtransform_dmma(EigArgs g, int mcap) {
-  extern __shared__ double sm[];
-  const int s = g.list[blockIdx.x];
-  if (g.only != nullptr && g.only[s] == 0) return;
-  const int n = g.nao[s];
-  const int m = g.all_vectors ? n : g.nvec[s];
-  const int nr = n - 2;
-  if (nr <= 0 || m <= 0) return;
-  constexpr int P = WB + 1;
-  const double* a = g.A + g.mat_off[s];
-  const double* tf = g.scratch + g.scratch_off[s] + wy_t_offset(n);
-  double* Z = g.Z + g.mat_off[s];
-  double* V = sm;                        // n x P
-  double* T = V + (size_t)n * P;         // WB x P
-  double* Y = T + WB * P;                // WB x mcap
-  double* Wm = Y + (size_t)WB * mcap;    // WB x mcap
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int gq = lane >> 2, tq = lane & 3;
-  const int nblk = (nr + WB - 1) / WB;
-  for (int it = 0; it < nblk; ++it) {
-    const int b = nblk - 1 - it;
-    const int i0 = b * WB;
-    const int k = min(WB, nr - i0);
-    const int L = n - i0 - 1;
-    __syncthreads();
-    load_wy_block(a, n, i0, k, L, V);
-    for (int idx = tid; idx < WB * WB; idx += blockDim.x)
-      T[(idx / WB) * P + (idx % WB)] = tf[(int64_t)b * WB * WB + idx];
-    __syncthreads();
-    // eigenvectors in chunks of mcap (the Y and W buffers' width): the count
-    // of a system's needed vectors is set on the device and can exceed the
-    // bucket's estimate
-    for (int j0 = 0; j0 < m; j0 += mcap) {
-      const int mc = min(mcap, m - j0);
-      const int jb_count = (mc + 7) / 8;
-      // Y = V^T Z over the block's rows
-      for (int jb = warp; jb < jb_count; jb += nw) {
-        double d[4][2];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) d[q][0] = d[q][1] = 0.0;
-        const int jl = jb * 8 + gq;
-        const double* z = Z + (int64_t)(j0 + jl) * n + i0 + 1;
-        // four K steps' loads of Z issued before their products (the
-        // products run in the same order as one step at a time)
-        for (int r0 = 0; r0 < L; r0 += 16) {
-          double bz[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int r = r0 + 4 * u + tq;
-            bz[u] = (jl < mc && r < L) ? z[r] : 0.0;
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int r = r0 + 4 * u + tq;
-            if (r0 + 4 * u < L) {
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const double av = r < L ? V[r * P + q * 8 + gq] : 0.0;
-                mma_f64(d[q], av, bz[u]);
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) Y[(q * 8 + gq) * mcap + jb * 8 + 2 * tq + h] = d[q][h];
-      }
-      __syncthreads();
-      // W = T Y (T upper triangular)
-      for (int idx = tid; idx < WB * mc; idx += blockDim.x) {
-        const int p = idx / mc, jj = idx - (idx / mc) * mc;
-        double acc = 0.0;
-        for (int q = p; q < WB; ++q) acc = fma(T[p * P + q], Y[q * mcap + jj], acc);
-        Wm[p * mcap + jj] = acc;
-      }
-      __syncthreads();
-      // Z^T tile (eigenvectors jb x rows rb) -= W^T V^T
-      const int rb_count = (L + 7) / 8;
-      for (int t = warp; t < jb_count * rb_count; t += nw) {
-        const int jb = t / rb_count, rb = t - (t / rb_count) * rb_count;
-        double d[2] = {0.0, 0.0};
-        const int jl = jb * 8 + gq, rr = rb * 8 + gq;
-        // the two elements of Z this lane updates, loaded before the products
-        double* z = Z + (int64_t)(j0 + jl) * n + i0 + 1;
-        double zold[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = rb * 8 + 2 * tq + h;
-          zold[h] = (jl < mc && r < L) ? z[r] : 0.0;
-        }
-#pragma unroll
-        for (int q0 = 0; q0 < WB; q0 += 4) {
-          const double aw = jl < mc ? Wm[(q0 + tq) * mcap + jl] : 0.0;
-          const double bv = rr < L ? V[rr * P + q0 + tq] : 0.0;
-          mma_f64(d, aw, bv);
-        }
-        if (jl < mc) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int r = rb * 8 + 2 * tq + h;
-            if (r < L) z[r] = zold[h] - d[h];
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-size_t backtransform_dmma_bytes(int n, int mcap) {
-  return ((size_t)n * (WB + 1) + WB * (WB + 1) + 2 * (size_t)WB * mcap) * sizeof(double);
-}
-
-void launch_wy_factor(const EigArgs& g, int count, int max_n, cudaStream_t stream) {
-  if (count == 0) return;
-  allow_max_dynamic_smem(k_wy_factor);
-  const int nblk = std::max(1, (max_n - 2 + WB - 1) / WB);
-  k_wy_factor<<<dim3(nblk, count), 256, wy_factor_bytes(max_n), stream>>>(g);
-}
-
-void launch_backtransform_wy(const EigArgs& g, int count, int max_n, int max_m, int want_m,
-                             cudaStream_t stream, bool factored) {
-  if (count == 0) return;
-  const size_t cap = allow_max_dynamic_smem(k_backtransform_wy<false>);
-  const size_t cap_s = allow_max_dynamic_smem(k_backtransform_wy<true>);
-  if (!factored) launch_wy_factor(g, count, max_n, stream);
-  // Few systems: split each system's vectors over CTAs, at least 8 vectors
-  // each, and keep each CTA's slice in shared memory when it fits.
-  const int sms = sm_count();
-  const int parts = count >= sms ? 1 : std::max(1, std::min((want_m + 7) / 8, 2 * sms / count));
-  const int per = (want_m + parts - 1) / parts;
-  const int wc = std::min(max_m, per);
-  const size_t staged = backtransform_wy_bytes(max_n, wc) + (size_t)per * max_n * sizeof(double) +
-                        ((size_t)max_n * (WB + 1) + WB * (WB + 1)) * sizeof(double);
-  if (parts > 1 && staged <= cap_s) {
-    k_backtransform_wy<true><<<dim3(parts, count), 256, staged, stream>>>(g, wc, per);
-    return;
-  }
-  // one CTA per system: the block products on the FP64 tensor cores
-  const int mcap = (want_m + 7) / 8 * 8;
-  const size_t capd = allow_max_dynamic_smem(k_backtransform_dmma);
-  if (parts == 1 && backtransform_dmma_bytes(max_n, mcap) <= capd) {
-    k_backtransform_dmma<<<count, 256, backtransform_dmma_bytes(max_n, mcap), stream>>>(g, mcap);
-    return;
-  }
-  (void)cap;
-  k_backtransform_wy<false><<<dim3(parts, count), 256, backtransform_wy_bytes(max_n, max_m), stream>>>(
-      g, max_m, 0);
-}
-
 // ---------------------------------------------------------------------------
 // Large systems (a 32-reflector block of n rows no longer fits in shared
-// memory): the same compact-WY algebra with the reflectors streamed through
-// shared memory in chunks of rows.
+// memory): the same T factors with the reflectors streamed through shared
+// memory in chunks of rows.
 // ---------------------------------------------------------------------------
 constexpr int kWyRows = 128;
 
@@ -1796,105 +1494,15 @@ __global__ void __launch_bounds__(256) k_wy_factor_rows(EigArgs g) {
 
 size_t wy_factor_rows_bytes() { return ((size_t)2 * kWyRows * (WB + 1) + 2 * WB * (WB + 1)) * sizeof(double); }
 
-// Back-transform of large systems: grid (vector slices of MC, systems); each
-// CTA keeps its MC eigenvectors in shared memory for the whole pass and, per
-// block (last to first), forms Y = V^T Z over row chunks, W = T Y, and
-// Z -= V W over the same chunks, the reflectors read from the matrix (L2).
-template <int MC>
-__global__ void __launch_bounds__(256) k_backtransform_rows(EigArgs g) {
-  extern __shared__ double sm[];
-  const int s = g.list[blockIdx.y];
-  if (g.only != nullptr && g.only[s] == 0) return;
-  const int n = g.nao[s];
-  const int mt = g.all_vectors ? n : g.nvec[s];
-  const int nr = n - 2;
-  if (nr <= 0) return;
-  const double* a = g.A + g.mat_off[s];
-  const double* tf = g.scratch + g.scratch_off[s] + wy_t_offset(n);
-  constexpr int P = WB + 1;
-  double* Z = sm;                          // MC x n
-  double* Vc = Z + (size_t)MC * n;         // kWyRows x P
-  double* T = Vc + kWyRows * P;            // WB x P
-  double* Y = T + WB * P;                  // WB x MC
-  double* W = Y + WB * MC;                 // WB x MC
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int nblk = (nr + WB - 1) / WB;
-  // slices of MC eigenvectors; the count of needed vectors is set on the
-  // device, so a CTA takes every gridDim.x-th slice until all are done
-  for (int jbeg = blockIdx.x * MC; jbeg < mt; jbeg += gridDim.x * MC) {
-    const int m = min(mt - jbeg, MC);
-    double* gZ = g.Z + g.mat_off[s] + (int64_t)jbeg * n;
-    __syncthreads();
-    for (int64_t k = tid; k < (int64_t)m * n; k += blockDim.x) Z[k] = gZ[k];
-    for (int it = 0; it < nblk; ++it) {
-      const int b = nblk - 1 - it;
-      const int i0 = b * WB;
-      const int k = min(WB, nr - i0);
-      const int L = n - i0 - 1;
-      for (int idx = tid; idx < WB * WB; idx += blockDim.x)
-        T[(idx / WB) * P + (idx % WB)] = tf[(int64_t)b * WB * WB + idx];
-      for (int idx = tid; idx < WB * MC; idx += blockDim.x) Y[idx] = 0.0;
-      // Y = V^T Z: lane = reflector, warps over this CTA's vectors
-      for (int r0 = 0; r0 < L; r0 += kWyRows) {
-        const int rc = min(kWyRows, L - r0);
-        __syncthreads();
-        load_wy_rows(a, n, i0, k, r0, rc, Vc);
-        __syncthreads();
-        for (int j = warp; j < m; j += nw) {
-          const double* z = Z + (int64_t)j * n + i0 + 1 + r0;
-          double acc = 0.0;
-          for (int r = 0; r < rc; ++r) acc = fma(Vc[r * P + lane], z[r], acc);
-          Y[lane * MC + j] += acc;
-        }
-      }
-      __syncthreads();
-      // W = T Y (T upper triangular)
-      for (int idx = tid; idx < WB * MC; idx += blockDim.x) {
-        const int p = idx / MC, j = idx - (idx / MC) * MC;
-        double acc = 0.0;
-        for (int q = p; q < WB; ++q) acc = fma(T[p * P + q], Y[q * MC + j], acc);
-        W[idx] = acc;
-      }
-      // Z -= V W
-      for (int r0 = 0; r0 < L; r0 += kWyRows) {
-        const int rc = min(kWyRows, L - r0);
-        __syncthreads();
-        load_wy_rows(a, n, i0, k, r0, rc, Vc);
-        __syncthreads();
-        for (int idx = tid; idx < rc * m; idx += blockDim.x) {
-          const int j = idx / rc, r = idx - (idx / rc) * rc;
-          const int qmax = min(k, r0 + r + 1);
-          double acc = 0.0;
-          for (int q = 0; q < qmax; ++q) acc = fma(Vc[r * P + q], W[q * MC + j], acc);
-          Z[(int64_t)j * n + i0 + 1 + r0 + r] -= acc;
-        }
-      }
-      __syncthreads();
-    }
-    for (int64_t k = tid; k < (int64_t)m * n; k += blockDim.x) gZ[k] = Z[k];
-  }
-}
-
-template <int MC>
-size_t backtransform_rows_bytes(int n) {
-  return ((size_t)MC * n + kWyRows * (WB + 1) + WB * (WB + 1) + 2 * WB * MC) * sizeof(double);
-}
-
-void launch_backtransform_rows(const EigArgs& g, int count, int max_n, int want_m, cudaStream_t stream) {
+void launch_wy_factor(const EigArgs& g, int count, int max_n, cudaStream_t stream) {
   if (count == 0) return;
   const int nblk = std::max(1, (max_n - 2 + WB - 1) / WB);
-  const size_t capf = allow_max_dynamic_smem(k_wy_factor_rows);
-  (void)capf;
-  k_wy_factor_rows<<<dim3(nblk, count), 256, wy_factor_rows_bytes(), stream>>>(g);
-  const size_t cap16 = allow_max_dynamic_smem(k_backtransform_rows<16>);
-  if (backtransform_rows_bytes<16>(max_n) <= cap16) {
-    k_backtransform_rows<16><<<dim3((want_m + 15) / 16, count), 256, backtransform_rows_bytes<16>(max_n),
-                               stream>>>(g);
-    return;
+  if (wy_factor_bytes(max_n) <= allow_max_dynamic_smem(k_wy_factor)) {
+    k_wy_factor<<<dim3(nblk, count), 256, wy_factor_bytes(max_n), stream>>>(g);
+  } else {
+    allow_max_dynamic_smem(k_wy_factor_rows);
+    k_wy_factor_rows<<<dim3(nblk, count), 256, wy_factor_rows_bytes(), stream>>>(g);
   }
-  const size_t cap4 = allow_max_dynamic_smem(k_backtransform_rows<4>);
-  (void)cap4;
-  k_backtransform_rows<4><<<dim3((want_m + 3) / 4, count), 256, backtransform_rows_bytes<4>(max_n), stream>>>(g);
 }
 
 // Loewdin weights s^-1/2 with the overlap condition guard; failed systems are flagged.
