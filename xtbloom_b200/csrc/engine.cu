@@ -260,7 +260,6 @@ struct Engine::Impl {
   int64_t nsys = 0, natoms = 0, nshells = 0, naos = 0, total_mat = 0, total_gam = 0, total_vec = 0,
           total_scr = 0, total_prim = 0;
   int max_n = 0, max_atoms = 0, max_shells = 0, max_dim = 0;
-  int64_t max_pairs = 0;
   std::vector<int32_t> h_nao, h_order;
   std::vector<double> h_nel_a, h_nel_b;
 
@@ -582,7 +581,6 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
       sh_spinw;
   int64_t shell = 0;
   int max_n = 0, max_atoms = 0, max_shells = 0, max_dim = 0;
-  int64_t max_pairs = 0;
   for (int64_t sy = 0; sy < B; ++sy) {
     shell_off[sy] = shell;
     ao_off[sy] = (int64_t)ao_sh.size();
@@ -696,7 +694,6 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
     max_atoms = std::max(max_atoms, na);
     max_shells = std::max(max_shells, ns);
     max_dim = std::max(max_dim, hb.nch[sy] * (g1 ? ns : ns + 9 * na));
-    max_pairs = std::max<int64_t>(max_pairs, (int64_t)na * (na + 1) / 2);
   }
   shell_off[B] = shell;
   ao_off[B] = (int64_t)ao_sh.size();
@@ -729,7 +726,6 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
   m.max_atoms = max_atoms;
   m.max_shells = max_shells;
   m.max_dim = max_dim;
-  m.max_pairs = max_pairs;
   m.h_nao = nao;
   m.h_order = order;
   m.h_nel_a = nel_a;
@@ -1256,7 +1252,7 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
   } while (0)
   // ---- geometry setup ----
   XTB_STAGE(kStSetup, 3,
-            launch_setup(t, list, nsys, m.max_atoms, m.max_pairs, m.max_shells, m.cn.as<double>(),
+            launch_setup(t, list, nsys, m.max_atoms, m.max_n, m.max_shells, m.cn.as<double>(),
                          m.cn_d4.as<double>(), m.mrad.as<double>(), m.dmrad.as<double>(),
                          m.S.as<double>(), m.D.as<double>(), m.Q.as<double>(), m.H0.as<double>(),
                          m.gam.as<double>(), m.total_mat, s);
@@ -1425,8 +1421,9 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
       }
       if (cnt == 0) return;
       // few systems: register-resident cluster kernel (latency); many: the
-      // shared-memory kernel, one CTA per system (throughput)
-      if (max_n <= tridiag_reg_max_n() && cnt * 8 <= sm_count() && !m.tridiag_smem)
+      // shared-memory kernel, one CTA per system (throughput).  The systems
+      // beside larger ones in a bucket stay on the shared-memory kernel.
+      if (bk.max_n <= tridiag_reg_max_n() && bk.count * 8 <= sm_count() && !m.tridiag_smem)
         launch_tridiag_reg(gb, gb.list, cnt, max_n, st);
       else
         launch_tridiag_smem(gb, gb.list, cnt, max_n, st);
@@ -1718,7 +1715,7 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
                    gemm(clist, m.C.as<double>(), dch_mat, m.C.as<double>(), dch_mat, m.W.as<double>(),
                         dnao, dnao, dnvec, true, m.occ_eps.as<double>(), fcc, true, nullptr, st);
                    combine(m.W.as<double>(), nullptr, fcount, st);
-                   launch_force_pairs(f, m.max_pairs, st));
+                   launch_force_pairs(f, m.max_atoms, st));
     }
     XTB_STAGE_ON(st, kStClassical, 1, launch_classical(f, m.max_atoms, m.max_shells, st));
     if (want_forces) XTB_STAGE_ON(st, kStCnChain, 2, launch_cn_chain(f, m.max_atoms, st));

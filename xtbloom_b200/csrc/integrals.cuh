@@ -66,40 +66,50 @@ __device__ __forceinline__ SphTerms sph_terms(int l, int m) {
 }
 
 // 1-D factors for one axis: O[e] = T[ek+e][eb] (e = 0..2) and, with GRAD,
-// G[e] = 2 a_k T[ek+e+1][eb] - (ek+e) T[ek+e-1][eb].
-template <bool GRAD>
+// G[e] = 2 a_k T[ek+e+1][eb] - (ek+e) T[ek+e-1][eb].  LM bounds both angular
+// momenta: the table ends there (for s and p shells it has a third of the
+// entries that d shells need); the entries are the same whatever LM.
+template <bool GRAD, int LM>
 __device__ __forceinline__ void axis_factors(double pa, double pb, double inv2p, double ak, int ek,
                                              int eb, double O[3], double G[3]) {
-  double T[6][3];
+  constexpr int NA = LM + (GRAD ? 4 : 3), NB = LM + 1;
+  double T[NA][NB];
 #pragma unroll
-  for (int a = 0; a < 6; ++a)
+  for (int a = 0; a < NA; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) T[a][b] = 0.0;
+    for (int b = 0; b < NB; ++b) T[a][b] = 0.0;
   T[0][0] = 1.0;
 #pragma unroll
-  for (int a = 1; a < 6; ++a) {
+  for (int a = 1; a < NA; ++a) {
     T[a][0] = pa * T[a - 1][0];
     if (a > 1) T[a][0] += (a - 1) * inv2p * T[a - 2][0];
   }
 #pragma unroll
-  for (int b = 1; b < 3; ++b) {
+  for (int b = 1; b < NB; ++b) {
     T[0][b] = pb * T[0][b - 1];
     if (b > 1) T[0][b] += (b - 1) * inv2p * T[0][b - 2];
 #pragma unroll
-    for (int a = 1; a < 6; ++a) {
+    for (int a = 1; a < NA; ++a) {
       T[a][b] = pa * T[a - 1][b] + b * inv2p * T[a - 1][b - 1];
-      if (a > 1) T[a][b] += (a - 1) * inv2p * T[a - 2][b];
+      // T[3][1]'s last product is also a term of T[2][2], so with d shells it
+      // is rounded before it is added; s and p shells keep that rounding
+      if (LM == 1 && a == 3 && b == 1) T[a][b] = __dadd_rn(T[a][b], __dmul_rn((a - 1) * inv2p, T[a - 2][b]));
+      else if (a > 1) T[a][b] += (a - 1) * inv2p * T[a - 2][b];
     }
   }
   // select the needed column entries without dynamic register indexing
-  double col[6];
+  double col[NA];
 #pragma unroll
-  for (int a = 0; a < 6; ++a) col[a] = (eb == 0) ? T[a][0] : ((eb == 1) ? T[a][1] : T[a][2]);
+  for (int a = 0; a < NA; ++a) {
+    col[a] = T[a][0];
+#pragma unroll
+    for (int b = 1; b < NB; ++b) col[a] = eb == b ? T[a][b] : col[a];
+  }
 #pragma unroll
   for (int e = 0; e < 3; ++e) {
     double o = 0.0, up = 0.0, dn = 0.0;
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
+    for (int a = 0; a < NA; ++a) {
       o = (a == ek + e) ? col[a] : o;
       up = (a == ek + e + 1) ? col[a] : up;
       dn = (a == ek + e - 1) ? col[a] : dn;
@@ -120,12 +130,12 @@ __device__ __forceinline__ void moment_powers(int m, int p[3]) {
 
 // Accumulate w * (S, 9 raw moments) [and derivatives w.r.t. the ket centre]
 // of one Cartesian pair.  v = R_ket - R_bra.
-template <bool GRAD>
+template <bool GRAD, int LM>
 __device__ __forceinline__ void cart_pair_acc(const int eb[3], const int ek[3], const double* ab,
                                               const double* cb, int npb, const double* ak,
                                               const double* ck, int npk, const double v[3],
                                               double w, double out[10], double dout[3][10]) {
-  const double r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+  const double r2 = fma(v[2], v[2], fma(v[0], v[0], v[1] * v[1]));
   for (int ik = 0; ik < npk; ++ik) {
     const double aK = ak[ik];
     for (int ib = 0; ib < npb; ++ib) {
@@ -138,78 +148,7 @@ __device__ __forceinline__ void cart_pair_acc(const int eb[3], const int ek[3], 
       double O[3][3], G[3][3];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
-        axis_factors<GRAD>(-v[c] * aB * inv, v[c] * aK * inv, inv2p, aK, ek[c], eb[c], O[c], G[c]);
-      out[0] += pref * O[0][0] * O[1][0] * O[2][0];
-      if (GRAD) {
-        dout[0][0] += pref * G[0][0] * O[1][0] * O[2][0];
-        dout[1][0] += pref * O[0][0] * G[1][0] * O[2][0];
-        dout[2][0] += pref * O[0][0] * O[1][0] * G[2][0];
-      }
-#pragma unroll
-      for (int m = 0; m < 9; ++m) {
-        int p[3];
-        moment_powers(m, p);
-        const double ox = O[0][p[0]], oy = O[1][p[1]], oz = O[2][p[2]];
-        out[1 + m] += pref * ox * oy * oz;
-        if (GRAD) {
-          dout[0][1 + m] += pref * G[0][p[0]] * oy * oz;
-          dout[1][1 + m] += pref * ox * G[1][p[1]] * oz;
-          dout[2][1 + m] += pref * ox * oy * G[2][p[2]];
-        }
-      }
-    }
-  }
-}
-
-// Primitive-pair factors of one shell pair at separation v (independent of
-// the Cartesian components): 1/(a_k + a_b), the screening exponent and, for
-// the pairs that pass the screen, exp(-est) and sqrt(1/(a_k + a_b)).  Index
-// ik * npb + ib.  cart_pair_acc_pp reads them instead of recomputing them
-// for every component pair; the values and the order of every product are
-// those of cart_pair_acc.
-constexpr int kPrimPairs = 36;   // shells with at most 6 primitives
-struct PrimPairs {
-  double inv[kPrimPairs], est[kPrimPairs], e[kPrimPairs], sinv[kPrimPairs];
-};
-__device__ __forceinline__ void prim_pairs(const double* ab, int npb, const double* ak, int npk,
-                                           const double v[3], PrimPairs& pp) {
-  // the contraction cart_pair_acc's r^2 compiles to, written out
-  const double r2 = fma(v[2], v[2], fma(v[0], v[0], v[1] * v[1]));
-  for (int ik = 0; ik < npk; ++ik) {
-    const double aK = ak[ik];
-    for (int ib = 0; ib < npb; ++ib) {
-      const double aB = ab[ib];
-      const int q = ik * npb + ib;
-      const double inv = 1.0 / (aK + aB);
-      const double est = aK * aB * r2 * inv;
-      pp.inv[q] = inv;
-      pp.est[q] = est;
-      if (est > kIntegralCutoff) continue;
-      pp.e[q] = exp(-est);
-      pp.sinv[q] = sqrt(inv);
-    }
-  }
-}
-
-template <bool GRAD>
-__device__ __forceinline__ void cart_pair_acc_pp(const int eb[3], const int ek[3], const double* ab,
-                                                 const double* cb, int npb, const double* ak,
-                                                 const double* ck, int npk, const double v[3],
-                                                 double w, const PrimPairs& pp, double out[10],
-                                                 double dout[3][10]) {
-  for (int ik = 0; ik < npk; ++ik) {
-    const double aK = ak[ik];
-    for (int ib = 0; ib < npb; ++ib) {
-      const double aB = ab[ib];
-      const int q = ik * npb + ib;
-      const double inv = pp.inv[q];
-      if (pp.est[q] > kIntegralCutoff) continue;
-      const double pref = w * pp.e[q] * kSqrtPi3 * inv * pp.sinv[q] * ck[ik] * cb[ib];
-      const double inv2p = 0.5 * inv;
-      double O[3][3], G[3][3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        axis_factors<GRAD>(-v[c] * aB * inv, v[c] * aK * inv, inv2p, aK, ek[c], eb[c], O[c], G[c]);
+        axis_factors<GRAD, LM>(-v[c] * aB * inv, v[c] * aK * inv, inv2p, aK, ek[c], eb[c], O[c], G[c]);
       out[0] += pref * O[0][0] * O[1][0] * O[2][0];
       if (GRAD) {
         dout[0][0] += pref * G[0][0] * O[1][0] * O[2][0];
@@ -245,8 +184,8 @@ __device__ __forceinline__ void make_traceless(double* m /* 6 raw: xx xy yy xz y
 // One spherical element pair (bra function mb of shell lb, ket function mk of
 // shell lk).  out = [S, Dx, Dy, Dz, Qxx, Qxy, Qyy, Qxz, Qyz, Qzz] with the
 // operator origin at the ket atom; dout[c][.] = derivatives w.r.t. R_ket[c].
-template <bool GRAD>
-__device__ __forceinline__ void sph_pair(int lb, int mb, int lk, int mk, const double* ab,
+template <bool GRAD, int LM>
+__device__ __forceinline__ void sph_pair_lm(int lb, int mb, int lk, int mk, const double* ab,
                                          const double* cb, int npb, const double* ak,
                                          const double* ck, int npk, const double v[3],
                                          double out[10], double dout[3][10]) {
@@ -263,7 +202,7 @@ __device__ __forceinline__ void sph_pair(int lb, int mb, int lk, int mk, const d
     for (int j = 0; j < tk.n; ++j) {
       int ek[3];
       cart_exponents(lk, tk.c[j], ek);
-      cart_pair_acc<GRAD>(eb, ek, ab, cb, npb, ak, ck, npk, v, tb.w[i] * tk.w[j], out, dout);
+      cart_pair_acc<GRAD, LM>(eb, ek, ab, cb, npb, ak, ck, npk, v, tb.w[i] * tk.w[j], out, dout);
     }
   }
   make_traceless(out + 4);
@@ -274,35 +213,15 @@ __device__ __forceinline__ void sph_pair(int lb, int mb, int lk, int mk, const d
   }
 }
 
-// sph_pair with the primitive-pair factors of prim_pairs.
 template <bool GRAD>
-__device__ __forceinline__ void sph_pair_pp(int lb, int mb, int lk, int mk, const double* ab,
-                                            const double* cb, int npb, const double* ak,
-                                            const double* ck, int npk, const double v[3],
-                                            const PrimPairs& pp, double out[10],
-                                            double dout[3][10]) {
-#pragma unroll
-  for (int i = 0; i < 10; ++i) {
-    out[i] = 0.0;
-    if (GRAD) { dout[0][i] = 0.0; dout[1][i] = 0.0; dout[2][i] = 0.0; }
-  }
-  const SphTerms tb = sph_terms(lb, mb);
-  const SphTerms tk = sph_terms(lk, mk);
-  for (int i = 0; i < tb.n; ++i) {
-    int eb[3];
-    cart_exponents(lb, tb.c[i], eb);
-    for (int j = 0; j < tk.n; ++j) {
-      int ek[3];
-      cart_exponents(lk, tk.c[j], ek);
-      cart_pair_acc_pp<GRAD>(eb, ek, ab, cb, npb, ak, ck, npk, v, tb.w[i] * tk.w[j], pp, out, dout);
-    }
-  }
-  make_traceless(out + 4);
-  if (GRAD) {
-    make_traceless(dout[0] + 4);
-    make_traceless(dout[1] + 4);
-    make_traceless(dout[2] + 4);
-  }
+__device__ __forceinline__ void sph_pair(int lb, int mb, int lk, int mk, const double* ab,
+                                         const double* cb, int npb, const double* ak,
+                                         const double* ck, int npk, const double v[3],
+                                         double out[10], double dout[3][10]) {
+  if (lb < 2 && lk < 2)
+    sph_pair_lm<GRAD, 1>(lb, mb, lk, mk, ab, cb, npb, ak, ck, npk, v, out, dout);
+  else
+    sph_pair_lm<GRAD, 2>(lb, mb, lk, mk, ab, cb, npb, ak, ck, npk, v, out, dout);
 }
 
 // Reverse element (ket row, bra column): the operator origin moves to the bra

@@ -22,132 +22,170 @@ __device__ __forceinline__ double lev(const DevTopo& t, int sh, const double* cn
   return t.sh_level[sh] - t.sh_kcn[sh] * cn[t.sh_atom[sh]];
 }
 
-__global__ void __launch_bounds__(128) k_force_pairs(ForceArgs f) {
+// H0 factor of a shell pair on different atoms and its pieces.
+struct PairFactors {
+  double avg, spat, dspat, fac;
+};
+__device__ __forceinline__ PairFactors pair_factors(const DevTopo& t, const double* cn, int bs, int ks, double r) {
+  PairFactors h;
+  h.avg = 0.5 * (lev(t, bs, cn) + lev(t, ks, cn));
+  const double ps = h0_pair_scale(t, bs, ks);
+  const double rr = sqrt(r / (t.at_rad[t.sh_atom[bs]] + t.at_rad[t.sh_atom[ks]]));
+  const double p1 = 1.0 + t.sh_shpoly[bs] * rr, p2 = 1.0 + t.sh_shpoly[ks] * rr;
+  h.spat = ps * p1 * p2;
+  h.dspat = ps * (t.sh_shpoly[bs] * p2 + t.sh_shpoly[ks] * p1) * rr / (2.0 * r);
+  h.fac = h.avg * h.spat;
+  return h;
+}
+
+// Integral gradients of the atoms B < A, one CTA per atom A.  The orbitals of
+// consecutive atoms are consecutive, so the CTA takes the rows of a run of
+// atoms B (at most kForceRows of them) and gives each thread one orbital pair
+// (row on B, column on A): the overlap and multipole integrals, their
+// derivatives and their contraction with the adjoints.  Then one thread per
+// atom pair adds its orbital pairs' contributions in shell order and posts the
+// pair's sums once.  A thread per atom pair did up to 81 contractions in a
+// row beside lanes that did one (C20 chain: 287 us; 2048 chains: 16.9 ms).
+constexpr int kForceRows = 128;
+constexpr int kForceThreads = 128;
+__global__ void __launch_bounds__(kForceThreads, 3) k_force_pairs(ForceArgs f) {
+  // per orbital pair: contribution to dE/dR_A and the overlap element; then
+  // the shell pairs' H0 factors
+  extern __shared__ double part[];
+  PairFactors* pf = reinterpret_cast<PairFactors*>(part + 4 * 9 * kForceRows);
   const DevTopo& t = f.t;
   const int s = f.list[blockIdx.y];
-  const int64_t a0 = t.atom_off[s], na = t.atom_off[s + 1] - a0;
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= na * (na + 1) / 2) return;
-  int64_t A = (int64_t)((sqrt(1.0 + 8.0 * (double)p) - 1.0) * 0.5);
-  while (A * (A + 1) / 2 > p) --A;
-  while ((A + 1) * (A + 2) / 2 <= p) ++A;
-  const int64_t B = p - A * (A + 1) / 2;
-  const int64_t gA = a0 + A, gB = a0 + B;
+  const int64_t a0 = t.atom_off[s];
+  const int na = (int)(t.atom_off[s + 1] - a0);
+  const int A = na - 1 - (int)blockIdx.x;   // the atoms with most partners first
+  if (A <= 0) return;
+  const int64_t gA = a0 + A;
   const int n = t.nao[s];
-  const int64_t mo = t.mat_off[s];
+  const int64_t mo = t.mat_off[s], o = t.ao_off[s];
   const double* P = f.P + mo;
   const double* W = f.W + mo;
   // unrestricted: the magnetisation is an overlap population too, so
   // P_alpha - P_beta with the spin potential enters the overlap adjoint
   const bool uhf = t.nch[s] == 2;
   const double* Pm = uhf ? f.Pm + mo : nullptr;
-  if (A == B) return;   // onsite blocks: k_force_onsite
-  const double v[3] = {t.pos[3 * gA] - t.pos[3 * gB], t.pos[3 * gA + 1] - t.pos[3 * gB + 1],
-                       t.pos[3 * gA + 2] - t.pos[3 * gB + 2]};
-  const double r = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
   const double* vdA = f.vd + 3 * gA;
-  const double* vdB = f.vd + 3 * gB;
   const double* vqA = f.vq + 6 * gA;
-  const double* vqB = f.vq + 6 * gB;
-  double g[3] = {0.0, 0.0, 0.0};
-  double cnA = 0.0, cnB = 0.0;
-  for (int ks = t.atom_sh[gA]; ks < t.atom_sh[gA + 1]; ++ks) {
-    const int lk = t.sh_l[ks];
-    const int npk = t.sh_np[ks];
-    const double* ak = t.p_alpha + t.sh_p0[ks];
-    const double* ck = t.p_coeff + t.sh_p0[ks];
-    const double vk = f.vsh[ks];
-    const double vmk = uhf ? f.vmag[ks] : 0.0;
-    for (int bs = t.atom_sh[gB]; bs < t.atom_sh[gB + 1]; ++bs) {
-      const int lb = t.sh_l[bs];
-      const int npb = t.sh_np[bs];
-      const double* ab = t.p_alpha + t.sh_p0[bs];
-      const double* cb = t.p_coeff + t.sh_p0[bs];
-      const double vb = f.vsh[bs];
-      const double vmb = uhf ? f.vmag[bs] : 0.0;
-      // H0 factor pieces
-      const double avg = 0.5 * (lev(t, bs, f.cn) + lev(t, ks, f.cn));
-      const double ps = h0_pair_scale(t, bs, ks);
-      const double rr = sqrt(r / (t.at_rad[gB] + t.at_rad[gA]));
-      const double p1 = 1.0 + t.sh_shpoly[bs] * rr, p2 = 1.0 + t.sh_shpoly[ks] * rr;
-      const double spat = ps * p1 * p2;
-      const double dspat = ps * (t.sh_shpoly[bs] * p2 + t.sh_shpoly[ks] * p1) * rr / (2.0 * r);
-      const double fac = avg * spat;
-      double bw = 0.0;
-      // the primitive-pair factors of this shell pair, shared by its 2l+1 x
-      // 2l'+1 function pairs (shells with more primitives recompute them)
-      const bool cached = npk * npb <= kPrimPairs;
-      PrimPairs pp;
-      if (cached) prim_pairs(ab, npb, ak, npk, v, pp);
-      for (int ib = 0; ib < 2 * lb + 1; ++ib) {
-        const int64_t row = t.sh_ao[bs] + ib;
-        for (int ik = 0; ik < 2 * lk + 1; ++ik) {
-          const int64_t col = t.sh_ao[ks] + ik;
-          const double Pv = P[row * n + col];
-          const double Wv = W[row * n + col];
-          double val[10], dv[3][10];
-          if (cached)
-            sph_pair_pp<true>(lb, ib, lk, ik, ab, cb, npb, ak, ck, npk, v, pp, val, dv);
-          else
-            sph_pair<true>(lb, ib, lk, ik, ab, cb, npb, ak, ck, npk, v, val, dv);
-          const double S = val[0];
-          bw += Pv * S;
-          double sA = 2.0 * (Pv * fac - Wv) - Pv * (vb + vk);
-          if (uhf) sA -= Pm[row * n + col] * (vmb + vmk);
-          double fD[3], rD[3], qadj[6], rQ[6];
+  auto first_ao = [&](int64_t g) { return t.sh_ao[t.atom_sh[g]]; };
+  const int colA = first_ao(gA);
+  const int ncol = (A + 1 < na ? first_ao(gA + 1) : n) - colA;
+  for (int B0 = 0; B0 < A;) {
+    const int row0 = first_ao(a0 + B0);
+    // the atom that holds row kForceRows of the run is the first one past it
+    const int B1 = row0 + kForceRows < colA ? (int)(t.ao_at[o + row0 + kForceRows] - a0) : A;
+    const int nrow = first_ao(a0 + B1) - row0;
+    const int ks0 = t.atom_sh[gA], nks = t.atom_sh[gA + 1] - ks0;
+    const int bs0 = t.atom_sh[a0 + B0], nbs = t.atom_sh[a0 + B1] - bs0;
+    for (int idx = threadIdx.x; idx < nks * nbs; idx += kForceThreads) {
+      const int ks = ks0 + idx / nbs, bs = bs0 + idx % nbs;
+      const int64_t gB = t.sh_atom[bs];
+      const double v[3] = {t.pos[3 * gA] - t.pos[3 * gB], t.pos[3 * gA + 1] - t.pos[3 * gB + 1],
+                           t.pos[3 * gA + 2] - t.pos[3 * gB + 2]};
+      pf[idx] = pair_factors(t, f.cn, bs, ks, sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nrow * ncol; idx += kForceThreads) {
+      const int row = row0 + idx % nrow, col = colA + idx / nrow;
+      const int ks = t.ao_sh[o + col], bs = t.ao_sh[o + row];
+      const int64_t gB = t.sh_atom[bs];
+      const double v[3] = {t.pos[3 * gA] - t.pos[3 * gB], t.pos[3 * gA + 1] - t.pos[3 * gB + 1],
+                           t.pos[3 * gA + 2] - t.pos[3 * gB + 2]};
+      const double* vdB = f.vd + 3 * gB;
+      const double* vqB = f.vq + 6 * gB;
+      const double vk = f.vsh[ks], vb = f.vsh[bs];
+      const double vmk = uhf ? f.vmag[ks] : 0.0, vmb = uhf ? f.vmag[bs] : 0.0;
+      const double fac = pf[(ks - ks0) * nbs + bs - bs0].fac;
+      const int64_t e = (int64_t)row * n + col;
+      const double Pv = P[e];
+      const double Wv = W[e];
+      double val[10], dv[3][10];
+      sph_pair<true>(t.sh_l[bs], row - t.sh_ao[bs], t.sh_l[ks], col - t.sh_ao[ks],
+                     t.p_alpha + t.sh_p0[bs], t.p_coeff + t.sh_p0[bs], t.sh_np[bs],
+                     t.p_alpha + t.sh_p0[ks], t.p_coeff + t.sh_p0[ks], t.sh_np[ks], v, val, dv);
+      const double S = val[0];
+      double sA = 2.0 * (Pv * fac - Wv) - Pv * (vb + vk);
+      if (uhf) sA -= Pm[e] * (vmb + vmk);
+      double fD[3], rD[3], qadj[6], rQ[6];
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            fD[c] = -Pv * vdA[c];
-            rD[c] = -Pv * vdB[c];
-          }
+      for (int c = 0; c < 3; ++c) {
+        fD[c] = -Pv * vdA[c];
+        rD[c] = -Pv * vdB[c];
+      }
 #pragma unroll
-          for (int c = 0; c < 6; ++c) {
-            rQ[c] = -Pv * vqB[c];
-            qadj[c] = -Pv * vqA[c] + rQ[c];
-          }
-          const double dsum = rQ[0] + rQ[2] + rQ[5];
-          const double axx = 1.5 * rQ[0] - 0.5 * dsum, axy = 1.5 * rQ[1];
-          const double ayy = 1.5 * rQ[2] - 0.5 * dsum, axz = 1.5 * rQ[3];
-          const double ayz = 1.5 * rQ[4], azz = 1.5 * rQ[5] - 0.5 * dsum;
-          const double x = v[0], y = v[1], z = v[2];
-          const double sadj = sA + rD[0] * x + rD[1] * y + rD[2] * z + axx * x * x + axy * x * y +
-                              ayy * y * y + axz * x * z + ayz * y * z + azz * z * z;
-          const double dadj[3] = {fD[0] + rD[0] + 2.0 * axx * x + axy * y + axz * z,
-                                  fD[1] + rD[1] + axy * x + 2.0 * ayy * y + ayz * z,
-                                  fD[2] + rD[2] + axz * x + ayz * y + 2.0 * azz * z};
-          const double Dx = val[1], Dy = val[2], Dz = val[3];
-          const double vadj[3] = {
-              rD[0] * S + axx * (2.0 * Dx + 2.0 * x * S) + axy * (Dy + y * S) + axz * (Dz + z * S),
-              rD[1] * S + axy * (Dx + x * S) + ayy * (2.0 * Dy + 2.0 * y * S) + ayz * (Dz + z * S),
-              rD[2] * S + axz * (Dx + x * S) + ayz * (Dy + y * S) + azz * (2.0 * Dz + 2.0 * z * S)};
+      for (int c = 0; c < 6; ++c) {
+        rQ[c] = -Pv * vqB[c];
+        qadj[c] = -Pv * vqA[c] + rQ[c];
+      }
+      const double dsum = rQ[0] + rQ[2] + rQ[5];
+      const double axx = 1.5 * rQ[0] - 0.5 * dsum, axy = 1.5 * rQ[1];
+      const double ayy = 1.5 * rQ[2] - 0.5 * dsum, axz = 1.5 * rQ[3];
+      const double ayz = 1.5 * rQ[4], azz = 1.5 * rQ[5] - 0.5 * dsum;
+      const double x = v[0], y = v[1], z = v[2];
+      const double sadj = sA + rD[0] * x + rD[1] * y + rD[2] * z + axx * x * x + axy * x * y +
+                          ayy * y * y + axz * x * z + ayz * y * z + azz * z * z;
+      const double dadj[3] = {fD[0] + rD[0] + 2.0 * axx * x + axy * y + axz * z,
+                              fD[1] + rD[1] + axy * x + 2.0 * ayy * y + ayz * z,
+                              fD[2] + rD[2] + axz * x + ayz * y + 2.0 * azz * z};
+      const double Dx = val[1], Dy = val[2], Dz = val[3];
+      const double vadj[3] = {
+          rD[0] * S + axx * (2.0 * Dx + 2.0 * x * S) + axy * (Dy + y * S) + axz * (Dz + z * S),
+          rD[1] * S + axy * (Dx + x * S) + ayy * (2.0 * Dy + 2.0 * y * S) + ayz * (Dz + z * S),
+          rD[2] * S + axz * (Dx + x * S) + ayz * (Dy + y * S) + azz * (2.0 * Dz + 2.0 * z * S)};
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            double acc = vadj[c] + sadj * dv[c][0];
+      for (int c = 0; c < 3; ++c) {
+        double acc = vadj[c] + sadj * dv[c][0];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) acc += dadj[k] * dv[c][1 + k];
+        for (int k = 0; k < 3; ++k) acc += dadj[k] * dv[c][1 + k];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) acc += qadj[k] * dv[c][4 + k];
-            g[c] += acc;
-          }
+        for (int k = 0; k < 6; ++k) acc += qadj[k] * dv[c][4 + k];
+        part[4 * idx + c] = acc;
+      }
+      part[4 * idx + 3] = S;
+    }
+    __syncthreads();
+    for (int B = B0 + threadIdx.x; B < B1; B += kForceThreads) {
+      const int64_t gB = a0 + B;
+      const double v[3] = {t.pos[3 * gA] - t.pos[3 * gB], t.pos[3 * gA + 1] - t.pos[3 * gB + 1],
+                           t.pos[3 * gA + 2] - t.pos[3 * gB + 2]};
+      const double r = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+      double g[3] = {0.0, 0.0, 0.0};
+      double cnA = 0.0, cnB = 0.0;
+      for (int ks = t.atom_sh[gA]; ks < t.atom_sh[gA + 1]; ++ks)
+        for (int bs = t.atom_sh[gB]; bs < t.atom_sh[gB + 1]; ++bs) {
+          const PairFactors& h = pf[(ks - ks0) * nbs + bs - bs0];
+          double bw = 0.0;
+          for (int ib = 0; ib < 2 * t.sh_l[bs] + 1; ++ib)
+            for (int ik = 0; ik < 2 * t.sh_l[ks] + 1; ++ik) {
+              const int row = t.sh_ao[bs] + ib, col = t.sh_ao[ks] + ik;
+              const double* q = part + 4 * ((col - colA) * nrow + row - row0);
+              bw += P[(int64_t)row * n + col] * q[3];
+#pragma unroll
+              for (int c = 0; c < 3; ++c) g[c] += q[c];
+            }
+          const double rad = 2.0 * bw * h.avg * h.dspat / r;
+          g[0] += rad * v[0];
+          g[1] += rad * v[1];
+          g[2] += rad * v[2];
+          cnB -= t.sh_kcn[bs] * bw * h.spat;
+          cnA -= t.sh_kcn[ks] * bw * h.spat;
+        }
+      if (f.want_grad) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          fix_add(&f.grad[3 * gA + c], g[c]);
+          fix_add(&f.grad[3 * gB + c], -g[c]);
         }
       }
-      const double rad = 2.0 * bw * avg * dspat / r;
-      g[0] += rad * v[0];
-      g[1] += rad * v[1];
-      g[2] += rad * v[2];
-      cnB -= t.sh_kcn[bs] * bw * spat;
-      cnA -= t.sh_kcn[ks] * bw * spat;
+      fix_add(&f.acn[gA], cnA);
+      fix_add(&f.acn[gB], cnB);
     }
+    __syncthreads();
+    B0 = B1;
   }
-  if (f.want_grad) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      fix_add(&f.grad[3 * gA + c], g[c]);
-      fix_add(&f.grad[3 * gB + c], -g[c]);
-    }
-  }
-  fix_add(&f.acn[gA], cnA);
-  fix_add(&f.acn[gB], cnB);
 }
 
 // Onsite CN adjoint of the shell levels: one thread per atom.
@@ -176,11 +214,12 @@ __global__ void k_force_onsite(ForceArgs f) {
   fix_add(&f.acn[gA], acc);
 }
 
-void launch_force_pairs(const ForceArgs& f, int64_t max_pairs, cudaStream_t stream) {
+void launch_force_pairs(const ForceArgs& f, int max_atoms, cudaStream_t stream) {
   if (f.count == 0) return;
-  const int tpb = 128;
-  dim3 grid((unsigned)((max_pairs + tpb - 1) / tpb), f.count);
-  k_force_pairs<<<grid, tpb, 0, stream>>>(f);
+  // at most nine orbitals and three shells on an atom
+  const size_t sm = (size_t)4 * 9 * kForceRows * sizeof(double) + 3 * kForceRows * sizeof(PairFactors);
+  allow_max_dynamic_smem(k_force_pairs);
+  k_force_pairs<<<dim3(max_atoms, f.count), kForceThreads, sm, stream>>>(f);
 }
 
 // ---------------------------------------------------------------------------

@@ -75,76 +75,58 @@ __global__ void k_coordination(DevTopo t, const int32_t* list, double* cn, doubl
   }
 }
 
-// One thread per atom pair (A >= B) of one system; writes every element of
-// the S, D, Q and H0 blocks (forward: rows on B, columns on A; reverse: rows
-// on A, columns on B, operator origin moved to B).
-__global__ void k_integrals(DevTopo t, const int32_t* list, const double* cn, double* S,
-                            double* D, double* Q, double* H0, int64_t total_mat) {
+// One thread per orbital pair (row <= col) of one system: the element and its
+// reverse of S, D, Q and H0 (forward: operator origin on the column's atom;
+// reverse: moved to the row's).  A thread carries one contraction of at most
+// 36 primitive pairs; a thread per atom pair carried up to 81 of them, so that
+// the pairs of heavy atoms set the time of their warp and of a small call
+// (one water 198 us, one C20 chain 266 us).
+__global__ void __launch_bounds__(128, 4) k_integrals(DevTopo t, const int32_t* list, const double* cn, double* S,
+                                                   double* D, double* Q, double* H0, int64_t total_mat) {
   const int s = list[blockIdx.y];
-  const int64_t a0 = t.atom_off[s], na = t.atom_off[s + 1] - a0;
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= na * (na + 1) / 2) return;
-  int64_t A = (int64_t)((sqrt(1.0 + 8.0 * (double)p) - 1.0) * 0.5);
-  while (A * (A + 1) / 2 > p) --A;
-  while ((A + 1) * (A + 2) / 2 <= p) ++A;
-  const int64_t B = p - A * (A + 1) / 2;
-  const int64_t gA = a0 + A, gB = a0 + B;
   const int n = t.nao[s];
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= (int64_t)n * (n + 1) / 2) return;
+  int64_t col, row;
+  col = (int64_t)((sqrt(1.0 + 8.0 * (double)p) - 1.0) * 0.5);
+  while (col * (col + 1) / 2 > p) --col;
+  while ((col + 1) * (col + 2) / 2 <= p) ++col;
+  row = p - col * (col + 1) / 2;
+  const int64_t o = t.ao_off[s];
+  const int ks = t.ao_sh[o + col], bs = t.ao_sh[o + row];
+  const int64_t gA = t.sh_atom[ks], gB = t.sh_atom[bs];
   const int64_t mo = t.mat_off[s];
   const double v[3] = {t.pos[3 * gA] - t.pos[3 * gB], t.pos[3 * gA + 1] - t.pos[3 * gB + 1],
                        t.pos[3 * gA + 2] - t.pos[3 * gB + 2]};
   const double r = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-  const bool same = (A == B);
-  for (int ks = t.atom_sh[gA]; ks < t.atom_sh[gA + 1]; ++ks) {
-    const int lk = t.sh_l[ks];
-    const int npk = t.sh_np[ks];
-    const double* ak = t.p_alpha + t.sh_p0[ks];
-    const double* ck = t.p_coeff + t.sh_p0[ks];
-    for (int bs = t.atom_sh[gB]; bs < t.atom_sh[gB + 1]; ++bs) {
-      if (same && bs > ks) continue;
-      const int lb = t.sh_l[bs];
-      const int npb = t.sh_np[bs];
-      const double* ab = t.p_alpha + t.sh_p0[bs];
-      const double* cb = t.p_coeff + t.sh_p0[bs];
-      const double fac = h0_factor(t, bs, ks, cn, r, same);
-      for (int ib = 0; ib < 2 * lb + 1; ++ib) {
-        const int64_t row = t.sh_ao[bs] + ib;
-        for (int ik = 0; ik < 2 * lk + 1; ++ik) {
-          if (bs == ks && ib > ik) continue;
-          const int64_t col = t.sh_ao[ks] + ik;
-          double val[10];
-          sph_pair<false>(lb, ib, lk, ik, ab, cb, npb, ak, ck, npk, v, val, nullptr);
-          const int64_t f = mo + row * n + col;
-          const int64_t rv = mo + col * n + row;
-          S[f] = val[0];
-          H0[f] = val[0] * fac;
+  const double fac = h0_factor(t, bs, ks, cn, r, gA == gB);
+  double val[10];
+  sph_pair<false>(t.sh_l[bs], (int)row - t.sh_ao[bs], t.sh_l[ks], (int)col - t.sh_ao[ks],
+                  t.p_alpha + t.sh_p0[bs], t.p_coeff + t.sh_p0[bs], t.sh_np[bs],
+                  t.p_alpha + t.sh_p0[ks], t.p_coeff + t.sh_p0[ks], t.sh_np[ks], v, val, nullptr);
+  const int64_t f = mo + row * n + col;
+  const int64_t rv = mo + col * n + row;
+  S[f] = val[0];
+  H0[f] = val[0] * fac;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) D[c * total_mat + f] = val[1 + c];
+  for (int c = 0; c < 3; ++c) D[c * total_mat + f] = val[1 + c];
 #pragma unroll
-          for (int c = 0; c < 6; ++c) Q[c * total_mat + f] = val[4 + c];
-          if (f == rv) continue;
-          if (bs == ks) {
-            // same shell on the same atom: exactly symmetric element pair
-            S[rv] = val[0];
-            H0[rv] = val[0] * fac;
+  for (int c = 0; c < 6; ++c) Q[c * total_mat + f] = val[4 + c];
+  if (f == rv) return;
+  // same shell on the same atom: exactly symmetric element pair
+  double rev[10];
+  if (bs != ks) {
+    shift_to_bra(v, val, rev);
+  } else {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) D[c * total_mat + rv] = val[1 + c];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) Q[c * total_mat + rv] = val[4 + c];
-            continue;
-          }
-          double rev[10];
-          shift_to_bra(v, val, rev);
-          S[rv] = val[0];
-          H0[rv] = val[0] * fac;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) D[c * total_mat + rv] = rev[1 + c];
-#pragma unroll
-          for (int c = 0; c < 6; ++c) Q[c * total_mat + rv] = rev[4 + c];
-        }
-      }
-    }
+    for (int c = 0; c < 10; ++c) rev[c] = val[c];
   }
+  S[rv] = val[0];
+  H0[rv] = val[0] * fac;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) D[c * total_mat + rv] = rev[1 + c];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) Q[c * total_mat + rv] = rev[4 + c];
 }
 
 // ES2 shell Coulomb matrix gamma_ij = 1/sqrt(r^2 + eta_ij^-2), onsite eta_ij,
@@ -174,7 +156,7 @@ __global__ void k_es2_gamma(DevTopo t, const int32_t* list, double* gam) {
 }
 
 void launch_setup(const DevTopo& t, const int32_t* list, int count, int max_atoms,
-                  int64_t max_pairs, int64_t max_shells, double* cn, double* cn_d4, double* mrad,
+                  int max_n, int64_t max_shells, double* cn, double* cn_d4, double* mrad,
                   double* dmrad, double* S, double* D, double* Q, double* H0, double* gam,
                   int64_t total_mat, cudaStream_t stream) {
   if (count == 0) return;
@@ -182,8 +164,8 @@ void launch_setup(const DevTopo& t, const int32_t* list, int count, int max_atom
   const size_t attr = allow_max_dynamic_smem(k_coordination);
   (void)attr;
   k_coordination<<<count, 256, sm, stream>>>(t, list, cn, cn_d4, mrad, dmrad);
-  const int tpb = 64;
-  dim3 g1((unsigned)((max_pairs + tpb - 1) / tpb), count);
+  const int tpb = 128;
+  dim3 g1((unsigned)(((int64_t)max_n * (max_n + 1) / 2 + tpb - 1) / tpb), count);
   k_integrals<<<g1, tpb, 0, stream>>>(t, list, cn, S, D, Q, H0, total_mat);
   dim3 g2((unsigned)((max_shells * max_shells + 255) / 256), count);
   k_es2_gamma<<<g2, 256, 0, stream>>>(t, list, gam);

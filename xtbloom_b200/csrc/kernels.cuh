@@ -148,7 +148,7 @@ constexpr int kMixedExtra = 10;
 constexpr int kMaxSplitIterations = 40;
 
 void launch_setup(const DevTopo& t, const int32_t* list, int count, int max_atoms,
-                  int64_t max_pairs, int64_t max_shells, double* cn, double* cn_d4, double* mrad,
+                  int max_n, int64_t max_shells, double* cn, double* cn_d4, double* mrad,
                   double* dmrad, double* S, double* D, double* Q, double* H0, double* gam,
                   int64_t total_mat, cudaStream_t stream);
 
@@ -294,7 +294,7 @@ struct ForceArgs {
   const int64_t* work_off;
 };
 
-void launch_force_pairs(const ForceArgs& f, int64_t max_pairs, cudaStream_t stream);
+void launch_force_pairs(const ForceArgs& f, int max_atoms, cudaStream_t stream);
 
 // external point charges (k_pc.cu)
 void launch_pc_potential(const DevTopo& t, const int32_t* list, int count, double* vpc,
