@@ -583,33 +583,93 @@ void launch_mulliken(const SccArgs& a, int max_n, cudaStream_t stream) {
 // ---------------------------------------------------------------------------
 // Energy functional from the raw populations, Broyden mixing, convergence.
 // ---------------------------------------------------------------------------
-__device__ bool cholesky_solve_small(double* B, double* c, int n) {
-  for (int r = 0; r < n; ++r) {
-    for (int col = 0; col <= r; ++col) {
-      double v = B[r * 8 + col];
-      for (int k = 0; k < col; ++k) v -= B[r * 8 + k] * B[col * 8 + k];
-      if (r == col) {
-        if (!(v > 0.0)) return false;
-        B[r * 8 + col] = sqrt(v);
-      } else {
-        B[r * 8 + col] = v / B[col * 8 + col];
-      }
+// One warp solves the n x n (n <= 8) symmetric system B x = c by Cholesky:
+// lane l holds rows l / 8 and l / 8 + 4 of column l % 8 of B (lower triangle
+// used), lane r < 8 holds c[r], and gets x[r].  Every element takes the
+// operations of the textbook row order, in that order; the columns' divisions
+// and updates run side by side instead of one after another.
+__device__ __forceinline__ bool cholesky_solve_warp(double b0, double b1, double& c, int n) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, col = lane & 7, r0 = lane >> 3, r1 = r0 + 4;
+  bool ok = true;
+  double diag = 1.0;   // lane r < 8: L[r][r]
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (k >= n) break;   // uniform over the warp
+    // element (r, k) sits in lane (r % 4) * 8 + k, register r / 4
+    const double d = __shfl_sync(kAll, k < 4 ? b0 : b1, (k & 3) * 8 + k);
+    if (!(d > 0.0)) ok = false;
+    const double l = sqrt(d);
+    if (lane == k) diag = l;
+    if (col == k) {
+      if (r0 > k) b0 = b0 / l;
+      if (r1 > k) b1 = b1 / l;
+    }
+    // the trailing elements lose L[r][k] L[col][k]
+    const double lr0 = __shfl_sync(kAll, b0, r0 * 8 + k), lr1 = __shfl_sync(kAll, b1, r0 * 8 + k);
+    const double c0 = __shfl_sync(kAll, b0, (col & 3) * 8 + k), c1 = __shfl_sync(kAll, b1, (col & 3) * 8 + k);
+    const double lc = col < 4 ? c0 : c1;
+    if (col > k) {
+      if (r0 >= col) b0 -= lr0 * lc;
+      if (r1 >= col) b1 -= lr1 * lc;
     }
   }
-  for (int r = 0; r < n; ++r) {
-    double v = c[r];
-    for (int k = 0; k < r; ++k) v -= B[r * 8 + k] * c[k];
-    c[r] = v / B[r * 8 + r];
+  // L y = c, then L^T x = y: lane r < 8 holds its right-hand side
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (k >= n) break;
+    const double e0 = __shfl_sync(kAll, b0, (lane & 3) * 8 + k), e1 = __shfl_sync(kAll, b1, (lane & 3) * 8 + k);
+    if (lane == k) c = c / diag;
+    const double y = __shfl_sync(kAll, c, k);
+    if (lane > k && lane < 8) c -= (lane < 4 ? e0 : e1) * y;
   }
-  for (int r = n - 1; r >= 0; --r) {
-    double v = c[r];
-    for (int k = r + 1; k < n; ++k) v -= B[k * 8 + r] * c[k];
-    c[r] = v / B[r * 8 + r];
+#pragma unroll
+  for (int r = 7; r >= 0; --r) {
+    if (r >= n) continue;
+    // row r needs x[k], k > r, in ascending order
+    double v = __shfl_sync(kAll, c, r);
+#pragma unroll
+    for (int k = r + 1; k < 8; ++k) {
+      const double e = __shfl_sync(kAll, k < 4 ? b0 : b1, (k & 3) * 8 + r);
+      const double x = __shfl_sync(kAll, c, k);
+      if (k < n) v -= e * x;
+    }
+    const double dr = __shfl_sync(kAll, diag, r);
+    if (lane == r) c = v / dr;
   }
-  return true;
+  return ok;
 }
 
-__global__ void __launch_bounds__(256) k_energy_mixer(SccArgs a) {
+// The totals over the warps of NV per-thread values: one pass and two
+// barriers, each value summed over its warp and then over the warps by the
+// same trees as block_sum.  scratch: NV * 32 doubles, then NV totals.
+template <int NV>
+__device__ __forceinline__ void block_sums(double (&v)[NV], double* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
+  __syncthreads();
+  if (lane == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) scratch[q * 32 + warp] = v[q];
+  }
+  __syncthreads();
+  for (int q = warp; q < NV; q += nw) {
+    const double t = warp_sum(lane < nw ? scratch[q * 32 + lane] : 0.0);
+    if (lane == 0) scratch[NV * 32 + q] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q] = scratch[NV * 32 + q];
+}
+
+// nine block sums, or 64 + the warps' 44 dot products
+constexpr int kMixerScratch = 64 + 8 * 44 + 8;
+static_assert(kMixerScratch >= 9 * 33, "block_sums of nine values");
+// Two CTAs per SM: at 190 registers a thread one fits, and 2048 chains spend
+// 11.2 instead of 6.9 ms of a call here.
+__global__ void __launch_bounds__(256, 2) k_energy_mixer(SccArgs a) {
   extern __shared__ double sm[];
   const DevTopo& t = a.t;
   const int s = a.list[blockIdx.x];
@@ -624,7 +684,7 @@ __global__ void __launch_bounds__(256) k_energy_mixer(SccArgs a) {
   double* raw = sm;                       // dim: [qsh, dip (3na), qp (6na)] (+ the same for m)
   double* qat = raw + dim;                // na
   double* w = qat + na;                   // 7 na
-  double* red = w + kMaxD4Refs * na;      // 64 + 8*64
+  double* red = w + kMaxD4Refs * na;      // kMixerScratch: sums of the block
   const int tid = threadIdx.x, bs = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nw = bs >> 5;
   for (int i = tid; i < ns; i += bs) raw[i] = t.sh_refocc[s0 + i] - a.pop_sh[s0 + i];
@@ -747,17 +807,20 @@ __global__ void __launch_bounds__(256) k_energy_mixer(SccArgs a) {
     }
   }
   // external point charges: E_pc = sum_s q_s V_s (potential fixed by the geometry)
-  double ep = 0.0;
+  double ep = 0.0, r2p = 0.0;
   if (t.vpc != nullptr)
     for (int i = tid; i < ns; i += bs) ep += raw[i] * t.vpc[s0 + i];
-  e2 = block_sum(e2, red);
-  e3 = block_sum(e3, red);
-  ea = block_sum(ea, red);
-  ed = block_sum(ed, red);
-  ep = block_sum(ep, red);
-  es = block_sum(es, red);
-  ef = block_sum(ef, red);
-  er = block_sum(er, red);
+  {
+    // the residual's square sum with them
+    const double* cur = a.mx_cur + t.vec_off[s];
+    for (int i = tid; i < dim; i += bs) {
+      const double r = raw[i] - cur[i];
+      r2p += r * r;
+    }
+    double v[9] = {e2, e3, ea, ed, ep, es, ef, er, r2p};
+    block_sums(v, red);
+    e2 = v[0], e3 = v[1], ea = v[2], ed = v[3], ep = v[4], es = v[5], ef = v[6], er = v[7], r2p = v[8];
+  }
   const double ecore = a.e_core[s];
   const int bch = t.beta_ch[s];
   const double ts = -a.kt * (a.entropy[s] + (bch >= 0 ? a.entropy[bch] : 0.0));
@@ -773,13 +836,7 @@ __global__ void __launch_bounds__(256) k_energy_mixer(SccArgs a) {
   double* uh = a.mx_u + v0 * M;
   double* om = a.mx_omega + (int64_t)s * M;
   const int it = a.iterations[s];
-  // residual norm
-  double r2p = 0.0;
-  for (int i = tid; i < dim; i += bs) {
-    const double r = raw[i] - cur[i];
-    r2p += r * r;
-  }
-  const double nrm = sqrt(block_sum(r2p, red));
+  const double nrm = sqrt(r2p);
   const double rms = nrm / sqrt((double)dim);
   __shared__ double s_c[8];
   __shared__ int s_hc, s_ok;
@@ -807,8 +864,8 @@ __global__ void __launch_bounds__(256) k_energy_mixer(SccArgs a) {
     const int first = it - hc + 1;
     int slot[8];
     for (int h = 0; h < 8; ++h) slot[h] = (h < hc) ? (first + h - 1) % M : 0;
-    double part[8 + 36];
-    for (int q = 0; q < 44; ++q) part[q] = 0.0;
+    double part[48];   // 8 + 36, padded for the halving below
+    for (int q = 0; q < 48; ++q) part[q] = 0.0;
     for (int i = tid; i < dim; i += bs) {
       const double r = raw[i] - cur[i];
       double dv[8];
@@ -823,10 +880,23 @@ __global__ void __launch_bounds__(256) k_energy_mixer(SccArgs a) {
       }
     }
     double* wsum = red + 64;   // [nw][44], then the 44 totals
+    // sums over the lanes, halving the values a lane carries at each exchange
+    // (warp_sum's tree: 48 exchanges instead of 220)
 #pragma unroll
-    for (int q = 0; q < 44; ++q) {
-      const double v = warp_sum(part[q]);
-      if (lane == 0) wsum[warp * 44 + q] = v;
+    for (int o = 16, h = 24; o >= 2; o >>= 1, h >>= 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int q = 0; q < h; ++q) {
+        const double send = up ? part[q] : part[q + h];
+        const double keep = up ? part[q + h] : part[q];
+        part[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    const int q0 = (lane & 16 ? 24 : 0) + (lane & 8 ? 12 : 0) + (lane & 4 ? 6 : 0) + (lane & 2 ? 3 : 0);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double v = part[q] + __shfl_xor_sync(0xffffffffu, part[q], 1);
+      if ((lane & 1) == 0 && q0 + q < 44) wsum[warp * 44 + q0 + q] = v;
     }
     __syncthreads();
     double* totals = red;      // the block sums above are done with red[0..32]
@@ -836,26 +906,27 @@ __global__ void __launch_bounds__(256) k_energy_mixer(SccArgs a) {
       totals[tid] = v;
     }
     __syncthreads();
-    if (tid == 0) {
-      double tot[44];
-      for (int q = 0; q < 44; ++q) tot[q] = totals[q];
-      double B[64], c[8];
-      int q = 8;
-      for (int h = 0; h < 8; ++h) {
-        for (int k = 0; k <= h; ++k) {
-          if (h < hc && k < hc) {
-            const double val = om[slot[h]] * om[slot[k]] * tot[q] + (h == k ? 1e-4 : 0.0);
-            B[h * 8 + k] = val;
-            B[k * 8 + h] = val;
-          }
-          ++q;
-        }
-        if (h < hc) c[h] = om[slot[h]] * tot[h];
+    if (warp == 0) {
+      // B (lower triangle) and c scaled by the weights, solved by this warp
+      const int col = lane & 7;
+      auto weight = [&](int h) { return h < hc ? om[(first + h - 1) % M] : 0.0; };
+      const double wl = weight(lane & 7);   // lane h < 8: omega_h
+      double b[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int row = (lane >> 3) + 4 * u;
+        const double wr = __shfl_sync(0xffffffffu, wl, row), wc = __shfl_sync(0xffffffffu, wl, col);
+        b[u] = row == col ? 1.0 : 0.0;
+        if (row < hc && col <= row)
+          b[u] = wr * wc * totals[8 + row * (row + 1) / 2 + col] + (row == col ? 1e-4 : 0.0);
       }
-      const bool ok = cholesky_solve_small(B, c, hc);
-      for (int h = 0; h < 8; ++h) s_c[h] = (h < hc) ? om[slot[h]] * c[h] : 0.0;
-      s_ok = ok ? 1 : 0;
-      s_hc = hc;
+      double c = lane < hc && lane < 8 ? wl * totals[lane] : 0.0;
+      const bool ok = cholesky_solve_warp(b[0], b[1], c, hc);
+      if (lane < 8) s_c[lane] = lane < hc ? wl * c : 0.0;
+      if (lane == 0) {
+        s_ok = ok ? 1 : 0;
+        s_hc = hc;
+      }
     }
     __syncthreads();
     hc = s_hc;
@@ -934,9 +1005,8 @@ void launch_energy_mixer(const SccArgs& a, int max_atoms, int max_shells, int ma
                          int first_iteration, cudaStream_t stream) {
   (void)first_iteration;
   if (a.count == 0) return;
-  const size_t sm = ((size_t)max_dim + (1 + kMaxD4Refs) * max_atoms + 64 + 8 * 44 + 8) * sizeof(double);
-  const size_t attr = allow_max_dynamic_smem(k_energy_mixer);
-  (void)attr;
+  const size_t sm = ((size_t)max_dim + (1 + kMaxD4Refs) * max_atoms + kMixerScratch) * sizeof(double);
+  allow_max_dynamic_smem(k_energy_mixer);
   k_energy_mixer<<<a.count, 256, sm, stream>>>(a);
 }
 
