@@ -1274,22 +1274,19 @@ __global__ void __launch_bounds__(128) k_inverse_iteration(EigArgs g, double ort
                                (uint32_t)s, 0, 128);
 }
 
-// Latency form for few systems: grid (parts, systems) of 16-thread CTAs whose
-// work vectors live in shared memory (5 n 16 doubles) instead of global
-// scratch; part p leads the clusters starting at p*16 + t, stepping 16 parts.
+// Latency form for few systems: grid (parts, systems) of T-thread CTAs whose
+// work vectors live in shared memory (5 n T doubles) instead of global
+// scratch; part p leads the clusters starting at p T + t, stepping T parts.
 constexpr int kInvSmemThreads = 16;
-__global__ void __launch_bounds__(kInvSmemThreads) k_inverse_iteration_smem(EigArgs g, double ortol_rel) {
+template <int T>
+__global__ void __launch_bounds__(T) k_inverse_iteration_smem(EigArgs g, double ortol_rel) {
   extern __shared__ double sm[];
   const int s = g.list[blockIdx.y];
   if (g.only != nullptr && g.only[s] == 0) return;
   const int64_t o = g.ao_off[s];
-  inverse_iteration_block<kInvSmemThreads>(g.d + o, g.e + o, g.eig + o, g.nao[s],
-                                           g.all_vectors ? g.nao[s] : g.nvec[s],
-                                           g.Z + g.mat_off[s], sm, ortol_rel, (uint32_t)s,
-                                           blockIdx.x * kInvSmemThreads,
-                                           gridDim.x * kInvSmemThreads);
+  inverse_iteration_block<T>(g.d + o, g.e + o, g.eig + o, g.nao[s], g.all_vectors ? g.nao[s] : g.nvec[s],
+                             g.Z + g.mat_off[s], sm, ortol_rel, (uint32_t)s, blockIdx.x * T, gridDim.x * T);
 }
-
 
 // ---------------------------------------------------------------------------
 // Compact-WY factors of the back-transform (k_backtransform.cu): the
@@ -1562,16 +1559,31 @@ void launch_eigvals(const EigArgs& g, int mode, double kt, int count, int max_n,
   k_tridiag_eigvals<<<count, 256, sm, stream>>>(g, mode, kt, 1, 8);
 }
 
+namespace {
+template <int T>
+bool try_inverse_iteration_smem(const EigArgs& g, int count, int max_n, int want_m, double ortol_rel,
+                                cudaStream_t stream) {
+  const size_t smem = (size_t)5 * max_n * T * sizeof(double);
+  if (smem > allow_max_dynamic_smem(k_inverse_iteration_smem<T>)) return false;
+  const int parts = std::max(1, (want_m + T - 1) / T);
+  // Below 16 threads a CTA fills its SM.  A vector then takes about a quarter
+  // of its time over global scratch (1200 orbitals: 0.2 against 0.8 ms), where
+  // each of 128 threads forms want_m / 128 vectors in turn.
+  const int64_t waves = ((int64_t)count * parts + sm_count() - 1) / sm_count();
+  if (T < kInvSmemThreads && waves > 3 * ((want_m + 127) / 128)) return false;
+  k_inverse_iteration_smem<T><<<dim3(parts, count), T, smem, stream>>>(g, ortol_rel);
+  return true;
+}
+}  // namespace
+
 void launch_inverse_iteration(const EigArgs& g, int count, int max_n, int want_m, double ortol_rel,
                               cudaStream_t stream) {
   if (count == 0) return;
-  const size_t smem = (size_t)5 * max_n * kInvSmemThreads * sizeof(double);
-  const size_t cap = allow_max_dynamic_smem(k_inverse_iteration_smem);
-  if (count < sm_count() && smem <= cap) {
-    const int parts = std::max(1, (want_m + kInvSmemThreads - 1) / kInvSmemThreads);
-    k_inverse_iteration_smem<<<dim3(parts, count), kInvSmemThreads, smem, stream>>>(g, ortol_rel);
+  if (count < sm_count() &&
+      (try_inverse_iteration_smem<kInvSmemThreads>(g, count, max_n, want_m, ortol_rel, stream) ||
+       try_inverse_iteration_smem<8>(g, count, max_n, want_m, ortol_rel, stream) ||
+       try_inverse_iteration_smem<4>(g, count, max_n, want_m, ortol_rel, stream)))
     return;
-  }
   k_inverse_iteration<<<count, 128, 0, stream>>>(g, ortol_rel);
 }
 
