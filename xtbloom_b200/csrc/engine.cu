@@ -66,6 +66,45 @@ bool upload(Dbuf& b, const std::vector<T>& v, cudaStream_t s) {
   return true;
 }
 
+// Pinned host memory that a topology is laid out in before it is copied to the
+// device: one block, grown to the largest topology of the engine, freed with it.
+struct PinnedArena {
+  char* base = nullptr;
+  size_t cap = 0, used = 0;
+  ~PinnedArena() {
+    if (base) cudaFreeHost(base);
+  }
+  PinnedArena() = default;
+  PinnedArena(const PinnedArena&) = delete;
+  PinnedArena& operator=(const PinnedArena&) = delete;
+  bool reset(size_t bytes) {
+    used = 0;
+    if (bytes <= cap) return true;
+    if (base) cudaFreeHost(base);
+    base = nullptr;
+    cap = 0;
+    if (cudaMallocHost(&base, bytes) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    cap = bytes;
+    return true;
+  }
+  static size_t padded(size_t bytes) { return (bytes + 63) / 64 * 64; }
+  template <class T>
+  T* take(size_t count) {   // within the reset size, by its computation
+    T* p = reinterpret_cast<T*>(base + used);
+    used += padded(count * sizeof(T));
+    return p;
+  }
+};
+
+template <class T>
+bool upload(Dbuf& b, const T* v, size_t count, cudaStream_t s) {
+  if (!b.reserve(count * sizeof(T))) return false;
+  return count == 0 || cudaMemcpyAsync(b.p, v, count * sizeof(T), cudaMemcpyHostToDevice, s) == cudaSuccess;
+}
+
 // STO-nG expansion (common/sto.cpp:20-123 of the reference, restated).
 bool sto_expand(int n, int l, int ng, double zeta, std::vector<double>& alpha,
                 std::vector<double>& coeff) {
@@ -257,6 +296,7 @@ struct Engine::Impl {
   // topology (host copies used for caching and sizes)
   HostBatch topo;
   bool topo_valid = false;
+  PinnedArena arena;
   int64_t nsys = 0, natoms = 0, nshells = 0, naos = 0, total_mat = 0, total_gam = 0, total_vec = 0,
           total_scr = 0, total_prim = 0;
   int max_n = 0, max_atoms = 0, max_shells = 0, max_dim = 0;
@@ -563,120 +603,189 @@ bool same_topology(const HostBatch& a, const HostBatch& b) {
          a.uhf == b.uhf && a.nch == b.nch && a.model == b.model;
 }
 
+// One element's atom and shell parameters of a model, primitives included.
+struct ElementShell {
+  int32_t l = 0, val = 0, p0 = 0, np = 0;   // p0: first primitive in the element tables
+  double level = 0, kcn = 0, shpoly = 0, zeta = 0, eta = 0, g3 = 0, refocc = 0;
+  double spinw[3] = {0, 0, 0};              // couplings to the atom's shells
+};
+struct Element {
+  bool ready = false;
+  int nsh = 0, nao = 0;
+  double en = 0, rad = 0, rcov = 0, mprad = 0, mpvcn = 0, dk = 0, qk = 0, rep_sa = 0, rep_z = 0, xbond = 0;
+  ElementShell sh[3];
+};
+
+// GFN1 (model/gfn1/basis.cpp, h0.cpp, es2.cpp, es3.cpp, repulsion.cpp,
+// coordination.cpp, halogen.cpp) or GFN2 parameters of element zi + 1; its
+// primitives are appended to p_alpha and p_coeff.
+bool make_element(const Engine::Impl& m, bool g1, int zi, Element& e, std::vector<double>& p_alpha,
+                  std::vector<double>& p_coeff) {
+  if (g1) {
+    e.en = kP_gfn1_en[zi];
+    e.rad = kP_gfn1_atomic_radius[zi];
+    e.rcov = kP_gfn1_covalent_radius[zi];
+    e.rep_sa = std::sqrt(kP_gfn1_arep[zi]);
+    e.rep_z = kP_gfn1_zeff[zi];
+    e.xbond = kP_gfn1_xbond[zi];
+  } else {
+    e.en = kP_gfn2_en[zi];
+    e.rad = kP_atomic_radii_angstrom[zi] * kAngstromToBohr;
+    e.rcov = (4.0 / 3.0) * kAngstromToBohr * kP_covalent_radii_angstrom[zi];
+    e.mprad = kP_gfn2_mprad[zi];
+    e.mpvcn = kP_gfn2_mpvcn[zi];
+    e.dk = kP_gfn2_dkernel[zi];
+    e.qk = kP_gfn2_qkernel[zi];
+    e.rep_sa = std::sqrt(kP_gfn2_arep[zi]);
+    e.rep_z = kP_gfn2_zeff[zi];
+  }
+  e.nsh = g1 ? kP_gfn1_nshell[zi] : kP_gfn2_nshell[zi];
+  int first_of_l[5] = {-1, -1, -1, -1, -1};
+  for (int k = 0; k < e.nsh; ++k) {
+    ElementShell& sh = e.sh[k];
+    const int q = 3 * zi + k;
+    sh.l = g1 ? kP_gfn1_shell_l[q] : kP_gfn2_shell_l[q];
+    const int pn = g1 ? kP_gfn1_shell_n[q] : kP_gfn2_shell_n[q];
+    const int ng = g1 ? kP_gfn1_shell_ngauss[q] : kP_gfn2_shell_ngauss[q];
+    sh.zeta = g1 ? kP_gfn1_shell_slater[q] : kP_gfn2_shell_slater[q];
+    std::vector<double> al, co;
+    if (!(g1 ? sto_expand_gfn1(pn, sh.l, ng, sh.zeta, al, co) : sto_expand(pn, sh.l, ng, sh.zeta, al, co)))
+      return false;
+    if (first_of_l[sh.l] >= 0) {
+      const ElementShell& f = e.sh[first_of_l[sh.l]];
+      std::vector<double> a1(p_alpha.begin() + f.p0, p_alpha.begin() + f.p0 + f.np);
+      std::vector<double> c1(p_coeff.begin() + f.p0, p_coeff.begin() + f.p0 + f.np);
+      orthogonalize_to_first(a1, c1, al, co);
+    } else {
+      first_of_l[sh.l] = k;
+    }
+    sh.p0 = (int32_t)p_alpha.size();
+    sh.np = (int32_t)al.size();
+    p_alpha.insert(p_alpha.end(), al.begin(), al.end());
+    p_coeff.insert(p_coeff.end(), co.begin(), co.end());
+    if (g1) {
+      // GFN1: levels and CN scales in eV (xTB's 27.21138505 conversion);
+      // third order per atom (no shell scaling)
+      sh.level = kP_gfn1_shell_level[q] * kEvToHartree;
+      sh.kcn = kP_gfn1_shell_kcn[q] * kEvToHartree;
+      sh.shpoly = kP_gfn1_shell_shpoly[q];
+      sh.eta = kP_gfn1_gam[zi] * kP_gfn1_shell_hubbard_scale[q];
+      sh.g3 = kP_gfn1_gam3[zi];
+      sh.val = kP_gfn1_shell_valence[q];
+      sh.refocc = kP_gfn1_shell_refocc[q];
+    } else {
+      sh.level = kP_gfn2_shell_level[q] * kEvToHartree;
+      sh.kcn = kP_gfn2_shell_kcn[q] * kEvToHartree;
+      sh.shpoly = kP_gfn2_shell_shpoly[q];
+      sh.eta = kP_gfn2_gam[zi] * kP_gfn2_shell_hubbard_scale[q];
+      sh.g3 = kP_gfn2_gam3[zi] * m.model_gfn2.es3_scale[sh.l];
+      sh.val = 1;
+      sh.refocc = kP_gfn2_shell_refocc[q];
+    }
+    e.nao += 2 * sh.l + 1;
+  }
+  // atom-local spin couplings W(l_row, l_col) (tblite element constants,
+  // ss sp pp sd pd dd), 3 per shell
+  for (int r = 0; r < e.nsh; ++r)
+    for (int k = 0; k < e.nsh; ++k) {
+      int l1 = e.sh[r].l, l2 = e.sh[k].l;
+      if (l1 > l2) std::swap(l1, l2);
+      const int idx = l1 == 0 ? (l2 == 0 ? 0 : (l2 == 1 ? 1 : 3)) : (l1 == 1 ? (l2 == 1 ? 2 : 4) : 5);
+      e.sh[r].spinw[k] = kP_spin_constants[6 * zi + idx];
+    }
+  e.ready = true;
+  return true;
+}
+
+// The parameters of an element are formed once and copied to its atoms (their
+// primitives are shared), into pinned memory that the copies to the device
+// read: expanding every shell of every atom anew and copying from pageable
+// vectors took 50 ms of a 265 ms call on 2048 new molecules.
 xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream_t s,
                                 std::string& error) {
   const int64_t B = hb.nsys;
   const int64_t N = hb.atom_off[B];
+  const bool g1 = hb.model == XTBLOOM_MODEL_GFN1_XTB;
+  std::vector<Element> elements(86);
+  std::vector<double> p_alpha, p_coeff;
+  int64_t shells = 0, aos = 0;
+  for (int64_t a = 0; a < N; ++a) {
+    Element& e = elements[hb.Z[a] - 1];
+    if (!e.ready && !make_element(m, g1, hb.Z[a] - 1, e, p_alpha, p_coeff)) {
+      error = "unsupported STO-nG shell in the parameter tables";
+      return XTBLOOM_STATUS_INTERNAL_ERROR;
+    }
+    shells += e.nsh;
+    aos += e.nao;
+  }
   std::vector<int64_t> atom_off = hb.atom_off, shell_off(B + 1), ao_off(B + 1), mat_off(B + 1),
                        gam_off(B + 1), vec_off(B + 1), scr_off(B + 1);
-  std::vector<int32_t> nao(B), Zv(hb.Z.begin(), hb.Z.end()), atom_sh(N + 1);
+  std::vector<int32_t> nao(B);
   std::vector<double> nel_a(B), nel_b(B), qmol(hb.qmol.begin(), hb.qmol.end());
-  std::vector<double> at_en(N), at_rad(N), at_rcov(N), at_mprad(N), at_mpvcn(N), at_dk(N), at_qk(N),
-      at_rep_sa(N), at_rep_z(N), at_xbond(N, 0.0);
-  std::vector<int32_t> sh_atom, sh_l, sh_ao, sh_p0, sh_np, ao_sh, ao_at, sh_val;
-  // GFN1 (model/gfn1/basis.cpp, h0.cpp, es2.cpp, es3.cpp, repulsion.cpp,
-  // coordination.cpp, halogen.cpp) or GFN2 element and shell parameters
-  const bool g1 = hb.model == XTBLOOM_MODEL_GFN1_XTB;
-  std::vector<double> sh_level, sh_kcn, sh_shpoly, sh_zeta, sh_eta, sh_g3, sh_refocc, p_alpha, p_coeff,
-      sh_spinw;
-  int64_t shell = 0;
+  PinnedArena& ar = m.arena;
+  const auto room = [](size_t count, size_t size) { return PinnedArena::padded(count * size); };
+  if (!ar.reset(10 * room(N, 8) + room(N, 4) + room(N + 1, 4) + 7 * room(shells, 8) + room(3 * shells, 8) +
+                6 * room(shells, 4) + 2 * room(aos, 4))) {
+    error = "pinned host allocation failed";
+    return XTBLOOM_STATUS_ALLOCATION_FAILED;
+  }
+  double *at_en = ar.take<double>(N), *at_rad = ar.take<double>(N), *at_rcov = ar.take<double>(N),
+         *at_mprad = ar.take<double>(N), *at_mpvcn = ar.take<double>(N), *at_dk = ar.take<double>(N),
+         *at_qk = ar.take<double>(N), *at_rep_sa = ar.take<double>(N), *at_rep_z = ar.take<double>(N),
+         *at_xbond = ar.take<double>(N);
+  int32_t *Zv = ar.take<int32_t>(N), *atom_sh = ar.take<int32_t>(N + 1);
+  double *sh_level = ar.take<double>(shells), *sh_kcn = ar.take<double>(shells),
+         *sh_shpoly = ar.take<double>(shells), *sh_zeta = ar.take<double>(shells),
+         *sh_eta = ar.take<double>(shells), *sh_g3 = ar.take<double>(shells),
+         *sh_refocc = ar.take<double>(shells), *sh_spinw = ar.take<double>(3 * shells);
+  int32_t *sh_atom = ar.take<int32_t>(shells), *sh_l = ar.take<int32_t>(shells),
+          *sh_ao = ar.take<int32_t>(shells), *sh_p0 = ar.take<int32_t>(shells),
+          *sh_np = ar.take<int32_t>(shells), *sh_val = ar.take<int32_t>(shells);
+  int32_t *ao_sh = ar.take<int32_t>(aos), *ao_at = ar.take<int32_t>(aos);
+  int64_t shell = 0, ao = 0;
   int max_n = 0, max_atoms = 0, max_shells = 0, max_dim = 0;
   for (int64_t sy = 0; sy < B; ++sy) {
     shell_off[sy] = shell;
-    ao_off[sy] = (int64_t)ao_sh.size();
+    ao_off[sy] = ao;
     int ao_local = 0;
     double nel = 0.0;
     for (int64_t a = atom_off[sy]; a < atom_off[sy + 1]; ++a) {
-      const int z = Zv[a];
-      const int zi = z - 1;
+      const Element& e = elements[hb.Z[a] - 1];
+      Zv[a] = hb.Z[a];
       atom_sh[a] = (int32_t)shell;
-      if (g1) {
-        at_en[a] = kP_gfn1_en[zi];
-        at_rad[a] = kP_gfn1_atomic_radius[zi];
-        at_rcov[a] = kP_gfn1_covalent_radius[zi];
-        at_mprad[a] = at_mpvcn[a] = at_dk[a] = at_qk[a] = 0.0;
-        at_rep_sa[a] = std::sqrt(kP_gfn1_arep[zi]);
-        at_rep_z[a] = kP_gfn1_zeff[zi];
-        at_xbond[a] = kP_gfn1_xbond[zi];
-      } else {
-        at_en[a] = kP_gfn2_en[zi];
-        at_rad[a] = kP_atomic_radii_angstrom[zi] * kAngstromToBohr;
-        at_rcov[a] = (4.0 / 3.0) * kAngstromToBohr * kP_covalent_radii_angstrom[zi];
-        at_mprad[a] = kP_gfn2_mprad[zi];
-        at_mpvcn[a] = kP_gfn2_mpvcn[zi];
-        at_dk[a] = kP_gfn2_dkernel[zi];
-        at_qk[a] = kP_gfn2_qkernel[zi];
-        at_rep_sa[a] = std::sqrt(kP_gfn2_arep[zi]);
-        at_rep_z[a] = kP_gfn2_zeff[zi];
-      }
-      const int nsh = g1 ? kP_gfn1_nshell[zi] : kP_gfn2_nshell[zi];
-      int first_of_l[5] = {-1, -1, -1, -1, -1};
-      for (int k = 0; k < nsh; ++k) {
-        const int l = g1 ? kP_gfn1_shell_l[3 * zi + k] : kP_gfn2_shell_l[3 * zi + k];
-        const int pn = g1 ? kP_gfn1_shell_n[3 * zi + k] : kP_gfn2_shell_n[3 * zi + k];
-        const int ng = g1 ? kP_gfn1_shell_ngauss[3 * zi + k] : kP_gfn2_shell_ngauss[3 * zi + k];
-        const double zeta = g1 ? kP_gfn1_shell_slater[3 * zi + k] : kP_gfn2_shell_slater[3 * zi + k];
-        std::vector<double> al, co;
-        if (!(g1 ? sto_expand_gfn1(pn, l, ng, zeta, al, co) : sto_expand(pn, l, ng, zeta, al, co))) {
-          error = "unsupported STO-nG shell in the parameter tables";
-          return XTBLOOM_STATUS_INTERNAL_ERROR;
+      at_en[a] = e.en;
+      at_rad[a] = e.rad;
+      at_rcov[a] = e.rcov;
+      at_mprad[a] = e.mprad;
+      at_mpvcn[a] = e.mpvcn;
+      at_dk[a] = e.dk;
+      at_qk[a] = e.qk;
+      at_rep_sa[a] = e.rep_sa;
+      at_rep_z[a] = e.rep_z;
+      at_xbond[a] = e.xbond;
+      for (int k = 0; k < e.nsh; ++k) {
+        const ElementShell& sh = e.sh[k];
+        sh_atom[shell] = (int32_t)a;
+        sh_l[shell] = sh.l;
+        sh_ao[shell] = ao_local;
+        sh_p0[shell] = sh.p0;
+        sh_np[shell] = sh.np;
+        sh_val[shell] = sh.val;
+        sh_level[shell] = sh.level;
+        sh_kcn[shell] = sh.kcn;
+        sh_shpoly[shell] = sh.shpoly;
+        sh_zeta[shell] = sh.zeta;
+        sh_eta[shell] = sh.eta;
+        sh_g3[shell] = sh.g3;
+        sh_refocc[shell] = sh.refocc;
+        for (int q = 0; q < 3; ++q) sh_spinw[3 * shell + q] = sh.spinw[q];
+        nel += sh.refocc;
+        for (int q = 0; q < 2 * sh.l + 1; ++q, ++ao) {
+          ao_sh[ao] = (int32_t)shell;
+          ao_at[ao] = (int32_t)a;
         }
-        if (first_of_l[l] >= 0) {
-          const int f = first_of_l[l];
-          std::vector<double> a1(p_alpha.begin() + sh_p0[f], p_alpha.begin() + sh_p0[f] + sh_np[f]);
-          std::vector<double> c1(p_coeff.begin() + sh_p0[f], p_coeff.begin() + sh_p0[f] + sh_np[f]);
-          orthogonalize_to_first(a1, c1, al, co);
-        } else {
-          first_of_l[l] = (int)shell;
-        }
-        sh_atom.push_back((int32_t)a);
-        sh_l.push_back(l);
-        sh_ao.push_back(ao_local);
-        sh_p0.push_back((int32_t)p_alpha.size());
-        sh_np.push_back((int32_t)al.size());
-        p_alpha.insert(p_alpha.end(), al.begin(), al.end());
-        p_coeff.insert(p_coeff.end(), co.begin(), co.end());
-        if (g1) {
-          // GFN1: levels and CN scales in eV (xTB's 27.21138505 conversion);
-          // third order per atom (no shell scaling)
-          sh_level.push_back(kP_gfn1_shell_level[3 * zi + k] * kEvToHartree);
-          sh_kcn.push_back(kP_gfn1_shell_kcn[3 * zi + k] * kEvToHartree);
-          sh_shpoly.push_back(kP_gfn1_shell_shpoly[3 * zi + k]);
-          sh_eta.push_back(kP_gfn1_gam[zi] * kP_gfn1_shell_hubbard_scale[3 * zi + k]);
-          sh_g3.push_back(kP_gfn1_gam3[zi]);
-          sh_val.push_back(kP_gfn1_shell_valence[3 * zi + k]);
-        } else {
-          sh_level.push_back(kP_gfn2_shell_level[3 * zi + k] * kEvToHartree);
-          sh_kcn.push_back(kP_gfn2_shell_kcn[3 * zi + k] * kEvToHartree);
-          sh_shpoly.push_back(kP_gfn2_shell_shpoly[3 * zi + k]);
-          sh_eta.push_back(kP_gfn2_gam[zi] * kP_gfn2_shell_hubbard_scale[3 * zi + k]);
-          sh_g3.push_back(kP_gfn2_gam3[zi] * m.model_gfn2.es3_scale[l]);
-          sh_val.push_back(1);
-        }
-        sh_zeta.push_back(zeta);
-        const double ro = g1 ? kP_gfn1_shell_refocc[3 * zi + k] : kP_gfn2_shell_refocc[3 * zi + k];
-        sh_refocc.push_back(ro);
-        nel += ro;
-        for (int q = 0; q < 2 * l + 1; ++q) {
-          ao_sh.push_back((int32_t)shell);
-          ao_at.push_back((int32_t)a);
-        }
-        ao_local += 2 * l + 1;
+        ao_local += 2 * sh.l + 1;
         ++shell;
-      }
-      // atom-local spin couplings W(l_row, l_col) (tblite element constants,
-      // ss sp pp sd pd dd), 3 per shell
-      for (int64_t r = atom_sh[a]; r < shell; ++r) {
-        for (int k = 0; k < 3; ++k) {
-          double wv = 0.0;
-          if (atom_sh[a] + k < shell) {
-            int l1 = sh_l[r], l2 = sh_l[atom_sh[a] + k];
-            if (l1 > l2) std::swap(l1, l2);
-            const int idx = l1 == 0 ? (l2 == 0 ? 0 : (l2 == 1 ? 1 : 3)) : (l1 == 1 ? (l2 == 1 ? 2 : 4) : 5);
-            wv = kP_spin_constants[6 * zi + idx];
-          }
-          sh_spinw.push_back(wv);
-        }
       }
     }
     const int na = (int)(atom_off[sy + 1] - atom_off[sy]);
@@ -696,7 +805,7 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
     max_dim = std::max(max_dim, hb.nch[sy] * (g1 ? ns : ns + 9 * na));
   }
   shell_off[B] = shell;
-  ao_off[B] = (int64_t)ao_sh.size();
+  ao_off[B] = ao;
   atom_sh[N] = (int32_t)shell;
   mat_off[0] = gam_off[0] = vec_off[0] = scr_off[0] = 0;
   for (int64_t sy = 0; sy < B; ++sy) {
@@ -789,7 +898,7 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
     }
     m.h_clist_cap = NC;
   }
-  if (!upload(m.nch, nchv, s) || !upload(m.beta_ch, beta, s) || !upload(m.sh_spinw, sh_spinw, s) ||
+  if (!upload(m.nch, nchv, s) || !upload(m.beta_ch, beta, s) || !upload(m.sh_spinw, sh_spinw, 3 * shells, s) ||
       !upload(m.ch_sys, ch_sys, s) || !upload(m.ch_sign, ch_sign, s) || !upload(m.ch_nao, ch_nao, s) ||
       !upload(m.ch_mat, ch_mat, s) || !upload(m.ch_ao, ch_ao, s) || !upload(m.ch_scr, ch_scr, s) ||
       !upload(m.ch_xoff, ch_xoff, s) || !upload(m.ch_nel_a, ch_nel_a, s) ||
@@ -797,28 +906,27 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
     error = "device allocation for the spin channels failed";
     return XTBLOOM_STATUS_ALLOCATION_FAILED;
   }
-  // the host vectors above must outlive their asynchronous uploads
-  cudaStreamSynchronize(s);
-
   bool ok = upload(m.atom_off, atom_off, s) && upload(m.shell_off, shell_off, s) &&
             upload(m.ao_off, ao_off, s) && upload(m.mat_off, mat_off, s) &&
             upload(m.gam_off, gam_off, s) && upload(m.vec_off, vec_off, s) &&
             upload(m.scr_off, scr_off, s) && upload(m.nao, nao, s) && upload(m.nel_a, nel_a, s) &&
-            upload(m.nel_b, nel_b, s) && upload(m.qmol, qmol, s) && upload(m.Z, Zv, s) &&
-            upload(m.atom_sh, atom_sh, s) && upload(m.at_en, at_en, s) &&
-            upload(m.at_rad, at_rad, s) && upload(m.at_rcov, at_rcov, s) &&
-            upload(m.at_mprad, at_mprad, s) && upload(m.at_mpvcn, at_mpvcn, s) &&
-            upload(m.at_dk, at_dk, s) && upload(m.at_qk, at_qk, s) &&
-            upload(m.at_rep_sa, at_rep_sa, s) && upload(m.at_rep_z, at_rep_z, s) &&
-            upload(m.at_xbond, at_xbond, s) && upload(m.sh_val, sh_val, s) &&
-            upload(m.sh_atom, sh_atom, s) && upload(m.sh_l, sh_l, s) && upload(m.sh_ao, sh_ao, s) &&
-            upload(m.sh_p0, sh_p0, s) && upload(m.sh_np, sh_np, s) &&
-            upload(m.sh_level, sh_level, s) && upload(m.sh_kcn, sh_kcn, s) &&
-            upload(m.sh_shpoly, sh_shpoly, s) && upload(m.sh_zeta, sh_zeta, s) &&
-            upload(m.sh_eta, sh_eta, s) && upload(m.sh_g3, sh_g3, s) &&
-            upload(m.sh_refocc, sh_refocc, s) && upload(m.p_alpha, p_alpha, s) &&
-            upload(m.p_coeff, p_coeff, s) && upload(m.ao_sh, ao_sh, s) &&
-            upload(m.ao_at, ao_at, s) && upload(m.order, order, s);
+            upload(m.nel_b, nel_b, s) && upload(m.qmol, qmol, s) && upload(m.Z, Zv, N, s) &&
+            upload(m.atom_sh, atom_sh, N + 1, s) && upload(m.at_en, at_en, N, s) &&
+            upload(m.at_rad, at_rad, N, s) && upload(m.at_rcov, at_rcov, N, s) &&
+            upload(m.at_mprad, at_mprad, N, s) && upload(m.at_mpvcn, at_mpvcn, N, s) &&
+            upload(m.at_dk, at_dk, N, s) && upload(m.at_qk, at_qk, N, s) &&
+            upload(m.at_rep_sa, at_rep_sa, N, s) && upload(m.at_rep_z, at_rep_z, N, s) &&
+            upload(m.at_xbond, at_xbond, N, s) && upload(m.sh_val, sh_val, shells, s) &&
+            upload(m.sh_atom, sh_atom, shells, s) && upload(m.sh_l, sh_l, shells, s) && upload(m.sh_ao, sh_ao, shells, s) &&
+            upload(m.sh_p0, sh_p0, shells, s) && upload(m.sh_np, sh_np, shells, s) &&
+            upload(m.sh_level, sh_level, shells, s) && upload(m.sh_kcn, sh_kcn, shells, s) &&
+            upload(m.sh_shpoly, sh_shpoly, shells, s) && upload(m.sh_zeta, sh_zeta, shells, s) &&
+            upload(m.sh_eta, sh_eta, shells, s) && upload(m.sh_g3, sh_g3, shells, s) &&
+            upload(m.sh_refocc, sh_refocc, shells, s) && upload(m.p_alpha, p_alpha, s) &&
+            upload(m.p_coeff, p_coeff, s) && upload(m.ao_sh, ao_sh, aos, s) &&
+            upload(m.ao_at, ao_at, aos, s) && upload(m.order, order, s);
+  // the vectors above and the pinned block must outlive their asynchronous copies
+  ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
   const size_t d8 = sizeof(double);
   const size_t mat = (size_t)m.total_mat * d8;
   const size_t cmat = (size_t)(m.total_mat + m.chan_mat) * d8;     // channel matrices
@@ -1025,7 +1133,7 @@ void Engine::invalidate_checkpoint() { impl_->ck_valid = false; }
 size_t Engine::device_bytes() const { return (size_t)std::max<int64_t>(0, impl_->ledger); }
 
 size_t Engine::host_bytes() const {
-  return 4 * sizeof(int32_t) + (size_t)impl_->h_list_cap * sizeof(int32_t) +
+  return 4 * sizeof(int32_t) + impl_->arena.cap + (size_t)impl_->h_list_cap * sizeof(int32_t) +
          (size_t)impl_->h_clist_cap * sizeof(int32_t);
 }
 
