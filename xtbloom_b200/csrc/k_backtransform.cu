@@ -19,7 +19,10 @@
 // What bounds it: with many systems the FP64 tensor pipe and the copies of V
 // (two CTAs per SM run each other's copies and products side by side); with
 // few, the chain of blocks (three barriers and two dependent products each),
-// which is why the next block's V is then copied ahead.
+// which is why the next block's V is then copied ahead.  Measured (B200): 361
+// systems of 212 orbitals and 106 vectors 376 us (757 us with the vectors in
+// global memory), one of 252 and 95 vectors 36 us (124 us with scalar FMAs),
+// twelve of 900 and 450 vectors 1.5 ms (8.0 ms).
 #include <algorithm>
 
 #include "kernels.cuh"
