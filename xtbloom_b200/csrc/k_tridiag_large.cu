@@ -414,20 +414,25 @@ int wide_clusters() {
 
 }  // namespace
 
+// Each shape against its own limit: the static shared memory beside the
+// vectors grows with G (16 CTAs leave 512 bytes less than eight).
+template <int G, int NW>
+static bool fits(int n) { return large_bytes<G, NW>(n) <= allow_max_dynamic_smem(k_tridiag_large<G, NW>); }
+
 // Largest system (the vectors and the warps' partial products of four warps
 // fill a CTA's shared memory).
-bool tridiag_large_fits(int max_n) { return large_bytes<8, 4>(max_n) <= allow_max_dynamic_smem(k_tridiag_large<8, 4>); }
+bool tridiag_large_fits(int max_n) { return fits<8, 4>(max_n); }
 
 void launch_tridiag_large(const EigArgs& g, const int32_t* list, int count, int max_n, cudaStream_t stream) {
   if (count == 0) return;
-  if (large_bytes<16, 8>(max_n) > allow_max_dynamic_smem(k_tridiag_large<8, 8>))
-    launch_cfg<8, 4>(g, list, count, max_n, stream);
   // a second set of eight CTAs pays from about 500 orbitals (600: 2.90 against
   // 3.20 ms; 360: 1.44 against 1.41) while every system still gets its SMs
-  else if (max_n > 480 && count <= wide_clusters<8>())
+  if (max_n > 480 && fits<16, 8>(max_n) && count <= wide_clusters<8>())
     launch_cfg<16, 8>(g, list, count, max_n, stream);
-  else
+  else if (fits<8, 8>(max_n))
     launch_cfg<8, 8>(g, list, count, max_n, stream);
+  else
+    launch_cfg<8, 4>(g, list, count, max_n, stream);   // above 2208 orbitals
 }
 
 }  // namespace xtb
