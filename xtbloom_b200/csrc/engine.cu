@@ -804,6 +804,18 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
     max_shells = std::max(max_shells, ns);
     max_dim = std::max(max_dim, hb.nch[sy] * (g1 ? ns : ns + 9 * na));
   }
+  // the largest system that every launch of the eigensolver has room for:
+  // larger ones are refused here, not by a launch in the middle of the call
+  const auto eigensolver_fits = [&](int n) {
+    return backtransform_fits(n) && (m.tridiag_smem ? tridiag_smem_fits(n) : tridiag_large_fits(n));
+  };
+  if (!eigensolver_fits(max_n)) {
+    int limit = max_n;
+    while (!eigensolver_fits(limit)) --limit;
+    error = "a system of " + std::to_string(max_n) + " orbitals exceeds the eigensolver's limit of " +
+            std::to_string(limit) + " on this device";
+    return XTBLOOM_STATUS_NOT_SUPPORTED;
+  }
   shell_off[B] = shell;
   ao_off[B] = ao;
   atom_sh[N] = (int32_t)shell;
@@ -1520,7 +1532,7 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
         int big = 0;
         while (big < cnt && m.h_ch_nao[first[big]] > tridiag_reg_max_n()) ++big;
         const int typical = m.h_ch_nao[first[big / 2]];
-        if (typical >= 600 || big <= 32 * (typical / 150)) {
+        if (typical >= 600 || big <= 32 * (typical / 150) || !tridiag_smem_fits(max_n)) {
           launch_tridiag_large(gb, gb.list, big, max_n, st);
           gb.list += big;
           cnt -= big;

@@ -299,6 +299,10 @@ void launch_rows(const EigArgs& g, int count, int n, int want, cudaStream_t stre
 
 }  // namespace
 
+// The row-chunk kernel takes every system up to here (2764 orbitals: eight
+// vectors beside two chunks of reflectors).
+bool backtransform_fits(int max_n) { return rows_bytes<8>(max_n) <= allow_max_dynamic_smem(k_backtransform_rows<8>); }
+
 void launch_backtransform(const EigArgs& g, int count, int max_n, int want_m, cudaStream_t stream) {
   if (count == 0) return;
   const size_t cap = std::min(allow_max_dynamic_smem(k_backtransform<8>), allow_max_dynamic_smem(k_backtransform<16>));

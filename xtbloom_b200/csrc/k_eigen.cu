@@ -878,6 +878,8 @@ __global__ void __launch_bounds__(NT) k_tridiag_prefix(EigArgs g, int nloc) {
 
 size_t tridiag_prefix_bytes(int n, int nt) { return ((4 + (size_t)nt / 32) * n + 64) * sizeof(double); }
 
+// Largest system of the single-CTA path (its prefix's vectors, 256 threads).
+bool tridiag_smem_fits(int max_n) { return tridiag_prefix_bytes(max_n, 256) <= allow_max_dynamic_smem(k_tridiag_prefix<256>); }
 
 // Largest trailing block the shared-memory kernel holds (227 KB per CTA).
 constexpr int kTridiagSmemMax = 228;

@@ -158,6 +158,7 @@ void launch_gemm_umma(const GemmArgs& g, bool transA, bool weighted, int tm, int
                       cudaStream_t stream);
 void launch_gemm(const GemmArgs& g, bool transA, bool weighted, int max_tiles, int count,
                  cudaStream_t stream, int width = 0);
+bool tridiag_smem_fits(int max_n);
 void launch_tridiag_smem(const EigArgs& g, const int32_t* list, int count, int max_n, cudaStream_t stream);
 // Register-resident cluster tridiagonalisation for systems with n <= tridiag_reg_max_n().
 int tridiag_reg_max_n();
@@ -179,6 +180,7 @@ void launch_inverse_iteration(const EigArgs& g, int count, int max_n, int want_m
 void launch_wy_factor(const EigArgs& g, int count, int max_n, cudaStream_t stream);
 // Back-transform of the tridiagonal eigenvectors, want_m of them a system at
 // the host's estimate (k_backtransform.cu).
+bool backtransform_fits(int max_n);
 void launch_backtransform(const EigArgs& g, int count, int max_n, int want_m, cudaStream_t stream);
 // Per-channel scratch of the eigensolver, in doubles: the inverse
 // iteration's work arrays (5 n per thread of a 128-thread block), then the
