@@ -2,12 +2,15 @@
 
 One SCC iteration of water clusters whose orbital counts sit at the edges of
 the cluster kernel's tiles (rows of 8, columns of 64, odd counts), for the
-launch shapes its rule picks (8 and 16 CTAs a system, more systems than
-clusters at once, small systems in the same call; at 2190 orbitals 16 CTAs no
-longer have the shared memory, above 2208 eight warps a CTA do not either).  The eigenvalues must be
-those of X H X (LAPACK), and the density, formed from the back-transformed
-vectors, LAPACK's: a backward-stable solver moves an occupied projector by
-about n eps ||A|| / gap, under 1e-11 here; 1e-9 leaves two orders.
+launch shapes its rule picks (8 and 16 CTAs a system, small systems in the
+same call; at 2190 orbitals 16 CTAs no longer have the shared memory, above 2208
+eight warps a CTA do not either), and for batches on both sides of the line to
+the single-CTA path: 33 x 262 are one wave of clusters, 60 x 360 two, more than
+run at once; 40 x 302 and 70 x 360 take the single CTAs, and 160 x 402, more
+than one wave of those, the clusters again.  The eigenvalues must be those of
+X H X (LAPACK), and the density, formed from the back-transformed vectors,
+LAPACK's: a backward-stable solver moves an occupied projector by about
+n eps ||A|| / gap, under 1e-11 here; 1e-9 leaves two orders.
 """
 from __future__ import annotations
 
@@ -41,7 +44,7 @@ def cluster(n):
 
 @pytest.mark.parametrize("sizes", [
     [258], [257, 259, 264], [320, 321, 319, 12], [384, 30, 200], [481], [600, 480], [1000], [2190], [2214],
-    [262] * 33, [258] * 9 + [90] * 40], ids=lambda s: "%dx%d" % (len(s), s[0]))
+    [262] * 33, [258] * 9 + [90] * 40, [360] * 60, [302] * 40, [360] * 70, [402] * 160], ids=lambda s: "%dx%d" % (len(s), s[0]))
 def test_eigenpairs_match_lapack(cuda_lib, sizes):
     mols = [cluster(n) for n in sizes]
     b = abi.ragged_from_lists([m[0] for m in mols], [m[1] for m in mols], [m[2] for m in mols])

@@ -1524,15 +1524,11 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
       const int32_t* first = hl + bk.start;
       // Systems beyond the register-resident kernel's size (the list is
       // n-descending): a cluster of SMs each, while that beats one SM each.
-      // About 32 clusters of eight CTAs run at once, so 32 k systems take k
-      // times one, against one wave of the single-CTA path: 1.2 against 1.5 ms
-      // at 258 orbitals, 1.8 against 4.1 ms at 360, 4.5 against 17.4 ms at 600;
-      // from there on the matrices of a full wave no longer fit L2 either.
       if (!m.tridiag_smem && max_n > tridiag_reg_max_n() && tridiag_large_fits(max_n)) {
         int big = 0;
         while (big < cnt && m.h_ch_nao[first[big]] > tridiag_reg_max_n()) ++big;
         const int typical = m.h_ch_nao[first[big / 2]];
-        if (typical >= 600 || big <= 32 * (typical / 150) || !tridiag_smem_fits(max_n)) {
+        if (tridiag_large_pays(typical, big) || !tridiag_smem_fits(max_n)) {
           launch_tridiag_large(gb, gb.list, big, max_n, st);
           gb.list += big;
           cnt -= big;

@@ -423,6 +423,47 @@ static bool fits(int n) { return large_bytes<G, NW>(n) <= allow_max_dynamic_smem
 // fill a CTA's shared memory).
 bool tridiag_large_fits(int max_n) { return fits<8, 4>(max_n); }
 
+// Systems run side by side, a cluster of eight CTAs each, two CTAs an SM (the
+// vectors of up to 1090 orbitals leave room for two).
+static int clusters_at_once() {
+  static std::mutex mu;
+  static std::map<int, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  allow_max_dynamic_smem(k_tridiag_large<8, 8>);
+  int active = 0;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = config<8, 8>(attr, 1, large_bytes<8, 8>(600), nullptr);
+  if (cudaOccupancyMaxActiveClusters(&active, k_tridiag_large<8, 8>, &cfg) != cudaSuccess || active < 1) {
+    (void)cudaGetLastError();
+    active = sm_count() / 8;
+  }
+  known.emplace(dev, active);
+  return active;
+}
+
+// Whether `count` systems of about n orbitals end sooner on clusters than one
+// to an SM.  Both sides take whole waves; a wave of the single-CTA path lasts
+// as long as about (n - 107) / 118 waves of clusters.  Measured, ms of the
+// clusters and of the single CTAs (33 systems fit one wave of clusters, 40 do
+// not; 148 fit one wave of single CTAs):
+//   258: 33 systems 1.18 / 1.52, 40: 2.25 / 1.52     300: 33 1.37 / 2.43, 40 2.68 / 2.43
+//   354: 64 3.70 / 3.96, 72 5.33 / 3.96              402: 64 4.59 / 5.69, 72 6.68 / 5.68
+//   450: 64 5.67 / 7.81, 72 8.15 / 7.81              504: 96 9.51 / 11.3, 128 12.7 / 12.2
+//   402: 149 11.4 / 11.5, 200 15.4 / 11.7            504: 149 15.6 / 23.1, 200 20.8 / 23.5
+// From 600 orbitals on the clusters win at every count tried (100: 13.4 / 19.7,
+// 148: 21.8 / 22.8, 200: 29.0 / 40.1): a wave of single CTAs no longer keeps
+// its matrices in L2.
+bool tridiag_large_pays(int n, int count) {
+  if (n >= 600) return true;
+  const int at_once = clusters_at_once(), sms = sm_count();
+  const int waves = (count + at_once - 1) / at_once, single = (count + sms - 1) / sms;
+  return 118 * waves <= (n - 107) * single;
+}
+
 void launch_tridiag_large(const EigArgs& g, const int32_t* list, int count, int max_n, cudaStream_t stream) {
   if (count == 0) return;
   // a second set of eight CTAs pays from about 500 orbitals (600: 2.90 against

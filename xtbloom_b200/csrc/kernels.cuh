@@ -166,6 +166,7 @@ void launch_tridiag_reg(const EigArgs& g, const int32_t* list, int count, int ma
 // Cluster tridiagonalisation with the matrix in global memory, for systems
 // above the register-resident kernel's size.
 bool tridiag_large_fits(int max_n);
+bool tridiag_large_pays(int n, int count);
 void launch_tridiag_large(const EigArgs& g, const int32_t* list, int count, int max_n, cudaStream_t stream);
 size_t tridiag_smem_bytes(int nl, int nt);
 int sm_count();   // multiprocessors of the current device (cached)
