@@ -1549,8 +1549,14 @@ xtbloom_status_t Engine::compute(const ComputeRequest& req, std::string& error) 
       launch_eigvals(sub(bk), mode, kt, bk.count, bk.max_n, bk.max_m + 4, st);
     };
     auto invit = [&](const Bucket& bk, cudaStream_t st) {
+      double work = 0.0;
+      for (int k = bk.start; k < bk.start + bk.count; ++k) {
+        const int c = hl[k], n = m.h_ch_nao[c];
+        const double want = std::ceil(std::max(m.h_ch_nel_a[c], m.h_ch_nel_b[c])) + 8;
+        work += (mode != 0 ? n : std::min<double>(want, n)) * n;
+      }
       launch_inverse_iteration(sub(bk), bk.count, bk.max_n,
-                               mode != 0 ? bk.max_n : std::min(bk.max_m + 4, bk.max_n), ortol_rel, st);
+                               mode != 0 ? bk.max_n : std::min(bk.max_m + 4, bk.max_n), work, ortol_rel, st);
     };
     // the T factors (launch_wy_factor) are formed before
     auto backtransform = [&](const Bucket& bk, cudaStream_t st) {

@@ -1563,28 +1563,32 @@ void launch_eigvals(const EigArgs& g, int mode, double kt, int count, int max_n,
 
 namespace {
 template <int T>
-bool try_inverse_iteration_smem(const EigArgs& g, int count, int max_n, int want_m, double ortol_rel,
-                                cudaStream_t stream) {
+bool try_inverse_iteration_smem(const EigArgs& g, int count, int max_n, int want_m, double work,
+                                double ortol_rel, cudaStream_t stream) {
   const size_t smem = (size_t)5 * max_n * T * sizeof(double);
   if (smem > allow_max_dynamic_smem(k_inverse_iteration_smem<T>)) return false;
   const int parts = std::max(1, (want_m + T - 1) / T);
-  // Below 16 threads a CTA fills its SM.  A vector then takes about a quarter
-  // of its time over global scratch (1200 orbitals: 0.2 against 0.8 ms), where
-  // each of 128 threads forms want_m / 128 vectors in turn.
-  const int64_t waves = ((int64_t)count * parts + sm_count() - 1) / sm_count();
-  if (T < kInvSmemThreads && waves > 3 * ((want_m + 127) / 128)) return false;
+  // A wave of these CTAs takes as long as 1 / 1.7 of a turn of 128 vectors over
+  // global scratch, from 366 to 1404 orbitals (ms a wave / a turn: 366 0.10 / 0.18,
+  // 600 0.16 / 0.27, 816 0.22 / 0.38, 1200 0.30 / 0.57); the waves from all systems'
+  // work, a vector's by its orbitals, the turns from the largest system alone.  On
+  // either side of the line, shared memory / scratch: 366 orbitals, 8 systems
+  // 0.20 / 0.36 and 24 0.58 / 0.36; 600, 12 systems 0.78 / 1.10 and 32 1.73 / 1.30;
+  // 1200, 8 systems 3.4 / 4.2 and 12 5.2 / 4.5.  (Sixteen threads stay, up to 363.)
+  const double waves = std::ceil(work / ((double)T * max_n * sm_count()));
+  if (T < kInvSmemThreads && waves > 1.7 * ((want_m + 127) / 128)) return false;
   k_inverse_iteration_smem<T><<<dim3(parts, count), T, smem, stream>>>(g, ortol_rel);
   return true;
 }
 }  // namespace
 
-void launch_inverse_iteration(const EigArgs& g, int count, int max_n, int want_m, double ortol_rel,
-                              cudaStream_t stream) {
+void launch_inverse_iteration(const EigArgs& g, int count, int max_n, int want_m, double work,
+                              double ortol_rel, cudaStream_t stream) {
   if (count == 0) return;
   if (count < sm_count() &&
-      (try_inverse_iteration_smem<kInvSmemThreads>(g, count, max_n, want_m, ortol_rel, stream) ||
-       try_inverse_iteration_smem<8>(g, count, max_n, want_m, ortol_rel, stream) ||
-       try_inverse_iteration_smem<4>(g, count, max_n, want_m, ortol_rel, stream)))
+      (try_inverse_iteration_smem<kInvSmemThreads>(g, count, max_n, want_m, work, ortol_rel, stream) ||
+       try_inverse_iteration_smem<8>(g, count, max_n, want_m, work, ortol_rel, stream) ||
+       try_inverse_iteration_smem<4>(g, count, max_n, want_m, work, ortol_rel, stream)))
     return;
   k_inverse_iteration<<<count, 128, 0, stream>>>(g, ortol_rel);
 }

@@ -174,8 +174,10 @@ int sm_count();   // multiprocessors of the current device (cached)
 // (mode 0): its occupied levels and eight above them.
 void launch_eigvals(const EigArgs& g, int mode, double kt, int count, int max_n, int max_levels,
                     cudaStream_t stream);
-void launch_inverse_iteration(const EigArgs& g, int count, int max_n, int want_m, double ortol_rel,
-                              cudaStream_t stream);
+// want_m: the most vectors a system of the launch needs; work: the sum over
+// its systems of the vectors each needs times its orbitals.
+void launch_inverse_iteration(const EigArgs& g, int count, int max_n, int want_m, double work,
+                              double ortol_rel, cudaStream_t stream);
 // T factors of the compact-WY back-transform; they need only the reflectors,
 // so they can be formed beside the eigenvalues and the inverse iteration.
 void launch_wy_factor(const EigArgs& g, int count, int max_n, cudaStream_t stream);
