@@ -139,6 +139,7 @@ struct DevTopo {
   // per AO (global)
   const int32_t* ao_sh;
   const int32_t* ao_at;
+  int32_t has_d;              // 1: a shell of the batch has l = 2
   // D4 reference tables
   const double* ref_cn;
   const double* ref_q;

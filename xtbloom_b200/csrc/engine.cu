@@ -300,6 +300,7 @@ struct Engine::Impl {
   int64_t nsys = 0, natoms = 0, nshells = 0, naos = 0, total_mat = 0, total_gam = 0, total_vec = 0,
           total_scr = 0, total_prim = 0;
   int max_n = 0, max_atoms = 0, max_shells = 0, max_dim = 0;
+  bool has_d = false;        // a shell of the batch has l = 2
   std::vector<int32_t> h_nao, h_order;
   std::vector<double> h_nel_a, h_nel_b;
 
@@ -443,6 +444,7 @@ struct Engine::Impl {
     t.nel_b = nel_b.as<double>();
     t.qmol = qmol.as<double>();
     t.nch = nch.as<int32_t>();
+    t.has_d = has_d ? 1 : 0;
     t.beta_ch = beta_ch.as<int32_t>();
     t.sh_spinw = sh_spinw.as<double>();
     t.efield = have_field ? efield.as<double>() : nullptr;
@@ -709,6 +711,7 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
   std::vector<Element> elements(86);
   std::vector<double> p_alpha, p_coeff;
   int64_t shells = 0, aos = 0;
+  bool has_d = false;
   for (int64_t a = 0; a < N; ++a) {
     Element& e = elements[hb.Z[a] - 1];
     if (!e.ready && !make_element(m, g1, hb.Z[a] - 1, e, p_alpha, p_coeff)) {
@@ -717,6 +720,7 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
     }
     shells += e.nsh;
     aos += e.nao;
+    for (int k = 0; k < e.nsh; ++k) has_d = has_d || e.sh[k].l == 2;
   }
   std::vector<int64_t> atom_off = hb.atom_off, shell_off(B + 1), ao_off(B + 1), mat_off(B + 1),
                        gam_off(B + 1), vec_off(B + 1), scr_off(B + 1);
@@ -847,6 +851,7 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
   m.max_atoms = max_atoms;
   m.max_shells = max_shells;
   m.max_dim = max_dim;
+  m.has_d = has_d;
   m.h_nao = nao;
   m.h_order = order;
   m.h_nel_a = nel_a;

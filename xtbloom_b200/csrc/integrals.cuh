@@ -65,6 +65,52 @@ __device__ __forceinline__ SphTerms sph_terms(int l, int m) {
   return t;
 }
 
+// Cost class of the contraction of two spherical functions: 0 for s and p
+// shells, with a d shell 1 and up by the number of Cartesian pairs.
+constexpr int kCostClasses = 7;
+__device__ __forceinline__ int cost_class(int lb, int mb, int lk, int mk) {
+  if (lb < 2 && lk < 2) return 0;
+  const auto terms = [](int l, int m) { return l < 2 ? 1 : (m == 2 ? 3 : (m == 4 ? 2 : 1)); };
+  const int pairs = terms(lb, mb) * terms(lk, mk);   // 1, 2, 3, 4, 6 or 9
+  return pairs <= 4 ? pairs : (pairs == 6 ? 5 : 6);
+}
+
+// Places of a block's items in an order by class, the most expensive first, so
+// that the lanes of a warp do alike contractions: with d shells a warp of
+// unsorted orbital pairs waits for its longest, nine Cartesian pairs, and runs
+// both table sizes.  Where an item lands within its class is not determined;
+// items must not depend on one another.  count: kCostClasses ints of shared
+// memory, zero on entry.  Call count_classes for every item (cls < 0: none),
+// by whole warps; after a barrier class_starts in one warp; after another
+// place for every item again.
+__device__ __forceinline__ void count_classes(int cls, int* count) {
+  for (int c = 0; c < kCostClasses; ++c) {
+    const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+    if (m != 0 && (threadIdx.x & 31) == 0) atomicAdd(count + c, __popc(m));
+  }
+}
+__device__ __forceinline__ void class_starts(int* count) {   // one thread
+  int at = 0;
+  for (int c = kCostClasses - 1; c >= 0; --c) {
+    const int k = count[c];
+    count[c] = at;
+    at += k;
+  }
+}
+__device__ __forceinline__ int place(int cls, int* count) {
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  for (int c = 0; c < kCostClasses; ++c) {
+    const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+    if (m == 0) continue;
+    int first = 0;
+    if (lane == 0) first = atomicAdd(count + c, __popc(m));
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (cls == c) at = first + __popc(m & ((1u << lane) - 1u));
+  }
+  return at;
+}
+
 // 1-D factors for one axis: O[e] = T[ek+e][eb] (e = 0..2) and, with GRAD,
 // G[e] = 2 a_k T[ek+e+1][eb] - (ek+e) T[ek+e-1][eb].  LM bounds both angular
 // momenta: the table ends there (for s and p shells it has a third of the

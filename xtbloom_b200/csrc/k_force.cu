@@ -46,6 +46,10 @@ __device__ __forceinline__ PairFactors pair_factors(const DevTopo& t, const doub
 // atom pair adds its orbital pairs' contributions in shell order and posts the
 // pair's sums once.  A thread per atom pair did up to 81 contractions in a
 // row beside lanes that did one (C20 chain: 287 us; 2048 chains: 16.9 ms).
+// Where a run has d shells its orbital pairs are dealt to the threads in order
+// of cost: as they lie, a warp holds pairs of one and of nine Cartesian pairs
+// (400 systems of four SiCl4: GFN2 8.4 -> 5.8 ms, GFN1 16.4 -> 10.7; a thread
+// per atom pair, all alike there, 6.4 and 12.8).
 constexpr int kForceRows = 128;
 constexpr int kForceThreads = 128;
 __global__ void __launch_bounds__(kForceThreads, 3) k_force_pairs(ForceArgs f) {
@@ -53,6 +57,9 @@ __global__ void __launch_bounds__(kForceThreads, 3) k_force_pairs(ForceArgs f) {
   // the shell pairs' H0 factors
   extern __shared__ double part[];
   PairFactors* pf = reinterpret_cast<PairFactors*>(part + 4 * 9 * kForceRows);
+  // batches with d shells: the orbital pairs of the run in order of their cost
+  uint16_t* order = reinterpret_cast<uint16_t*>(pf + 3 * kForceRows);
+  __shared__ int cost[kCostClasses];
   const DevTopo& t = f.t;
   const int s = f.list[blockIdx.y];
   const int64_t a0 = t.atom_off[s];
@@ -87,8 +94,34 @@ __global__ void __launch_bounds__(kForceThreads, 3) k_force_pairs(ForceArgs f) {
                            t.pos[3 * gA + 2] - t.pos[3 * gB + 2]};
       pf[idx] = pair_factors(t, f.cn, bs, ks, sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
     }
+    bool sorted = false;
+    if (t.has_d) {
+      auto cost_of = [&](int idx) {
+        if (idx >= nrow * ncol) return -1;
+        const int row = row0 + idx % nrow, col = colA + idx / nrow;
+        const int ks = t.ao_sh[o + col], bs = t.ao_sh[o + row];
+        return cost_class(t.sh_l[bs], row - t.sh_ao[bs], t.sh_l[ks], col - t.sh_ao[ks]);
+      };
+      const int rounds = (nrow * ncol + kForceThreads - 1) / kForceThreads;
+      if (threadIdx.x < kCostClasses) cost[threadIdx.x] = 0;
+      bool d = false;
+      for (int k = 0; k < rounds; ++k) d = d || cost_of(k * kForceThreads + threadIdx.x) > 0;
+      sorted = __syncthreads_or(d);
+      if (sorted) {
+        for (int k = 0; k < rounds; ++k) count_classes(cost_of(k * kForceThreads + threadIdx.x), cost);
+        __syncthreads();
+        if (threadIdx.x == 0) class_starts(cost);
+        __syncthreads();
+        for (int k = 0; k < rounds; ++k) {
+          const int idx = k * kForceThreads + threadIdx.x, c = cost_of(idx);
+          const int at = place(c, cost);
+          if (c >= 0) order[at] = (uint16_t)idx;
+        }
+      }
+    }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < nrow * ncol; idx += kForceThreads) {
+    for (int item = threadIdx.x; item < nrow * ncol; item += kForceThreads) {
+      const int idx = sorted ? order[item] : item;
       const int row = row0 + idx % nrow, col = colA + idx / nrow;
       const int ks = t.ao_sh[o + col], bs = t.ao_sh[o + row];
       const int64_t gB = t.sh_atom[bs];
@@ -217,7 +250,8 @@ __global__ void k_force_onsite(ForceArgs f) {
 void launch_force_pairs(const ForceArgs& f, int max_atoms, cudaStream_t stream) {
   if (f.count == 0) return;
   // at most nine orbitals and three shells on an atom
-  const size_t sm = (size_t)4 * 9 * kForceRows * sizeof(double) + 3 * kForceRows * sizeof(PairFactors);
+  const size_t sm = (size_t)4 * 9 * kForceRows * sizeof(double) + 3 * kForceRows * sizeof(PairFactors) +
+                    (f.t.has_d ? 9 * kForceRows * sizeof(uint16_t) : 0);
   allow_max_dynamic_smem(k_force_pairs);
   k_force_pairs<<<dim3(max_atoms, f.count), kForceThreads, sm, stream>>>(f);
 }

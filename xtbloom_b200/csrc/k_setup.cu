@@ -78,20 +78,52 @@ __global__ void k_coordination(DevTopo t, const int32_t* list, double* cn, doubl
 // One thread per orbital pair (row <= col) of one system: the element and its
 // reverse of S, D, Q and H0 (forward: operator origin on the column's atom;
 // reverse: moved to the row's).  A thread carries one contraction of at most
-// 36 primitive pairs; a thread per atom pair carried up to 81 of them, so that
+// 49 primitive pairs; a thread per atom pair carried up to 81 of them, so that
 // the pairs of heavy atoms set the time of their warp and of a small call
-// (one water 198 us, one C20 chain 266 us).
-__global__ void __launch_bounds__(128, 4) k_integrals(DevTopo t, const int32_t* list, const double* cn, double* S,
-                                                   double* D, double* Q, double* H0, int64_t total_mat) {
+// (one water 198 us, one C20 chain 266 us).  Where the CTA's pairs have d shells
+// they are dealt to its threads in order of cost, as in k_force_pairs (400
+// systems of four SiCl4: GFN2 5.4 -> 4.1 ms, GFN1 10.1 -> 7.2; a thread per atom
+// pair 4.9 and 8.8).
+constexpr int kIntegralThreads = 128;
+__global__ void __launch_bounds__(kIntegralThreads, 4) k_integrals(DevTopo t, const int32_t* list, const double* cn,
+                                                                   double* S, double* D, double* Q, double* H0,
+                                                                   int64_t total_mat) {
   const int s = list[blockIdx.y];
   const int n = t.nao[s];
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= (int64_t)n * (n + 1) / 2) return;
-  int64_t col, row;
-  col = (int64_t)((sqrt(1.0 + 8.0 * (double)p) - 1.0) * 0.5);
-  while (col * (col + 1) / 2 > p) --col;
-  while ((col + 1) * (col + 2) / 2 <= p) ++col;
-  row = p - col * (col + 1) / 2;
+  const int64_t p0 = (int64_t)blockIdx.x * kIntegralThreads, pairs = (int64_t)n * (n + 1) / 2;
+  if (p0 >= pairs) return;   // uniform over the CTA
+  int64_t p = p0 + threadIdx.x, col, row;
+  auto locate = [&] {
+    col = (int64_t)((sqrt(1.0 + 8.0 * (double)p) - 1.0) * 0.5);
+    while (col * (col + 1) / 2 > p) --col;
+    while ((col + 1) * (col + 2) / 2 <= p) ++col;
+    row = p - col * (col + 1) / 2;
+  };
+  if (t.has_d) {
+    __shared__ int count[kCostClasses];
+    __shared__ uint8_t order[kIntegralThreads];
+    if (threadIdx.x < kCostClasses) count[threadIdx.x] = 0;
+    order[threadIdx.x] = 255;   // no pair
+    int cls = -1;
+    if (p < pairs) {
+      locate();
+      const int ks = t.ao_sh[t.ao_off[s] + col], bs = t.ao_sh[t.ao_off[s] + row];
+      cls = cost_class(t.sh_l[bs], (int)row - t.sh_ao[bs], t.sh_l[ks], (int)col - t.sh_ao[ks]);
+    }
+    if (__syncthreads_or(cls > 0)) {   // a pair with a d shell
+      count_classes(cls, count);
+      __syncthreads();
+      if (threadIdx.x == 0) class_starts(count);
+      __syncthreads();
+      const int at = place(cls, count);
+      if (cls >= 0) order[at] = (uint8_t)threadIdx.x;
+      __syncthreads();
+      if (order[threadIdx.x] == 255) return;
+      p = p0 + order[threadIdx.x];
+    }
+  }
+  if (p >= pairs) return;
+  locate();
   const int64_t o = t.ao_off[s];
   const int ks = t.ao_sh[o + col], bs = t.ao_sh[o + row];
   const int64_t gA = t.sh_atom[ks], gB = t.sh_atom[bs];
@@ -164,9 +196,8 @@ void launch_setup(const DevTopo& t, const int32_t* list, int count, int max_atom
   const size_t attr = allow_max_dynamic_smem(k_coordination);
   (void)attr;
   k_coordination<<<count, 256, sm, stream>>>(t, list, cn, cn_d4, mrad, dmrad);
-  const int tpb = 128;
-  dim3 g1((unsigned)(((int64_t)max_n * (max_n + 1) / 2 + tpb - 1) / tpb), count);
-  k_integrals<<<g1, tpb, 0, stream>>>(t, list, cn, S, D, Q, H0, total_mat);
+  dim3 g1((unsigned)(((int64_t)max_n * (max_n + 1) / 2 + kIntegralThreads - 1) / kIntegralThreads), count);
+  k_integrals<<<g1, kIntegralThreads, 0, stream>>>(t, list, cn, S, D, Q, H0, total_mat);
   dim3 g2((unsigned)((max_shells * max_shells + 255) / 256), count);
   k_es2_gamma<<<g2, 256, 0, stream>>>(t, list, gam);
 }
