@@ -21,6 +21,7 @@
 #include <numeric>
 
 #include "kernels.cuh"
+#include "pinned_arena.h"
 
 namespace xtb {
 namespace {
@@ -66,38 +67,16 @@ bool upload(Dbuf& b, const std::vector<T>& v, cudaStream_t s) {
   return true;
 }
 
-// Pinned host memory that a topology is laid out in before it is copied to the
-// device: one block, grown to the largest topology of the engine, freed with it.
-struct PinnedArena {
-  char* base = nullptr;
-  size_t cap = 0, used = 0;
-  ~PinnedArena() {
-    if (base) cudaFreeHost(base);
+struct CudaPinned {
+  static void* allocate(size_t bytes) {
+    void* p = nullptr;
+    if (cudaMallocHost(&p, bytes) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    return nullptr;
   }
-  PinnedArena() = default;
-  PinnedArena(const PinnedArena&) = delete;
-  PinnedArena& operator=(const PinnedArena&) = delete;
-  bool reset(size_t bytes) {
-    used = 0;
-    if (bytes <= cap) return true;
-    if (base) cudaFreeHost(base);
-    base = nullptr;
-    cap = 0;
-    if (cudaMallocHost(&base, bytes) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return false;
-    }
-    cap = bytes;
-    return true;
-  }
-  static size_t padded(size_t bytes) { return (bytes + 63) / 64 * 64; }
-  template <class T>
-  T* take(size_t count) {   // within the reset size, by its computation
-    T* p = reinterpret_cast<T*>(base + used);
-    used += padded(count * sizeof(T));
-    return p;
-  }
+  static void release(void* p) { cudaFreeHost(p); }
 };
+using PinnedArena = HostArena<CudaPinned>;
 
 template <class T>
 bool upload(Dbuf& b, const T* v, size_t count, cudaStream_t s) {
@@ -730,7 +709,7 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
   const auto room = [](size_t count, size_t size) { return PinnedArena::padded(count * size); };
   if (!ar.reset(10 * room(N, 8) + room(N, 4) + room(N + 1, 4) + 7 * room(shells, 8) + room(3 * shells, 8) +
                 6 * room(shells, 4) + 2 * room(aos, 4))) {
-    error = "pinned host allocation failed";
+    error = "host allocation for the topology failed";
     return XTBLOOM_STATUS_ALLOCATION_FAILED;
   }
   double *at_en = ar.take<double>(N), *at_rad = ar.take<double>(N), *at_rcov = ar.take<double>(N),
@@ -910,7 +889,7 @@ xtbloom_status_t build_topology(Engine::Impl& m, const HostBatch& hb, cudaStream
     if (m.h_clist) cudaFreeHost(m.h_clist);
     m.h_clist = nullptr;
     if (cudaMallocHost(&m.h_clist, NC * sizeof(int32_t)) != cudaSuccess) {
-      error = "pinned host allocation failed";
+      error = "host allocation for the topology failed";
       return XTBLOOM_STATUS_ALLOCATION_FAILED;
     }
     m.h_clist_cap = NC;
@@ -1150,7 +1129,7 @@ void Engine::invalidate_checkpoint() { impl_->ck_valid = false; }
 size_t Engine::device_bytes() const { return (size_t)std::max<int64_t>(0, impl_->ledger); }
 
 size_t Engine::host_bytes() const {
-  return 4 * sizeof(int32_t) + impl_->arena.cap + (size_t)impl_->h_list_cap * sizeof(int32_t) +
+  return 4 * sizeof(int32_t) + impl_->arena.capacity() + (size_t)impl_->h_list_cap * sizeof(int32_t) +
          (size_t)impl_->h_clist_cap * sizeof(int32_t);
 }
 
