@@ -44,7 +44,8 @@ def cluster(n):
 
 @pytest.mark.parametrize("sizes", [
     [258], [257, 259, 264], [320, 321, 319, 12], [384, 30, 200], [481], [600, 480], [1000], [2190], [2214],
-    [262] * 33, [258] * 9 + [90] * 40, [360] * 60, [302] * 40, [360] * 70, [402] * 160], ids=lambda s: "%dx%d" % (len(s), s[0]))
+    [262] * 33, [258] * 9 + [90] * 40, [360] * 60, [302] * 40, [360] * 70, [402] * 160,
+    [600, 594, 588, 577, 569, 560, 552, 537, 520, 513, 504, 481]], ids=lambda s: "%dx%d" % (len(s), s[0]))
 def test_eigenpairs_match_lapack(cuda_lib, sizes):
     mols = [cluster(n) for n in sizes]
     b = abi.ragged_from_lists([m[0] for m in mols], [m[1] for m in mols], [m[2] for m in mols])
