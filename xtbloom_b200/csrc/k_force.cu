@@ -46,6 +46,10 @@ __device__ __forceinline__ PairFactors pair_factors(const DevTopo& t, const doub
 // atom pair adds its orbital pairs' contributions in shell order and posts the
 // pair's sums once.  A thread per atom pair did up to 81 contractions in a
 // row beside lanes that did one (C20 chain: 287 us; 2048 chains: 16.9 ms).
+// What bounds it now: 168 registers, 12 warps an SM, and the two barriers of a
+// run (512 hetero-alkanes, 2.4 ms: issue active 33 % of cycles, FP64 pipe 25 %;
+// 3.3 warps wait at a barrier per issued instruction, 2.0 for a fixed latency,
+// 1.7 for memory).  260 bytes of spill stores a thread.
 // Where a run has d shells its orbital pairs are dealt to the threads in order
 // of cost: as they lie, a warp holds pairs of one and of nine Cartesian pairs
 // (400 systems of four SiCl4: GFN2 8.4 -> 5.8 ms, GFN1 16.4 -> 10.7; a thread

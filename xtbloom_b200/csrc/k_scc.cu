@@ -667,8 +667,9 @@ __device__ __forceinline__ void block_sums(double (&v)[NV], double* scratch) {
 // nine block sums, or 64 + the warps' 44 dot products
 constexpr int kMixerScratch = 64 + 8 * 44 + 8;
 static_assert(kMixerScratch >= 9 * 33, "block_sums of nine values");
-// Two CTAs per SM: at 190 registers a thread one fits, and 2048 chains spend
-// 11.2 instead of 6.9 ms of a call here.
+// Two CTAs per SM: without the bound a thread has 190 registers, one CTA fits,
+// and 2048 chains spend 10.4 instead of 5.9 ms of a call here.  The bound costs
+// 92 bytes of spill stores a thread (one C20 chain 0.60 ms against 0.59).
 __global__ void __launch_bounds__(256, 2) k_energy_mixer(SccArgs a) {
   extern __shared__ double sm[];
   const DevTopo& t = a.t;

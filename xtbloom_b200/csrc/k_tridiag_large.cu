@@ -23,13 +23,18 @@
 // every CTA during step o, so its reflector is written during step o+1.
 //
 // What bounds it: a column costs about 3.5 us of barriers and dependent sums
-// (n = 258) and, above about 500 orbitals, the instructions of (2).  Measured
-// (B200, one system): n = 360 1.41 ms, 600 2.90 ms, 900 5.8 ms, 1200 9.7 ms;
-// the single-CTA prefix (k_tridiag_prefix + k_tridiag_smem) took 4.1, 17.4 and,
-// at 1200, 126 ms.  A butterfly per unit instead of per row block: 38 ms
-// instead of 13 ms at n = 1200 with eight CTAs.  Eight warps a CTA, two CTAs an
-// SM: sixteen warps take the same time alone and leave no room for a second
-// system (30 systems of 258: 1.19 ms instead of 2.4 ms).
+// (n = 258) and, above about 500 orbitals, the units of (2): their dependent
+// multiply-adds and L2 loads, which the two warps a scheduler do not hide (8
+// systems of 600 to 1200 orbitals: issue active 32 % of cycles, FP64 pipe 12 %,
+// L2 12 %; per issued instruction 1.4 waits for a fixed latency, 1.1 for L2, 0.8
+// at barriers).  Measured (B200, one system): n = 360 1.41 ms, 600 2.90 ms, 900
+// 5.8 ms, 1200 9.7 ms, 2100 33 ms; with four warps a CTA, where eight have no
+// room, 2214 100 ms; the single-CTA prefix (k_tridiag_prefix + k_tridiag_smem)
+// took 4.1, 17.4 and, at 1200, 126 ms.  A butterfly per unit instead of per row
+// block: 38 ms instead of 13 ms at n = 1200 with eight CTAs.  Eight warps a CTA,
+// two CTAs an SM: sixteen warps take the same time alone and leave no room for
+// a second system (30 systems of 258: 1.19 ms instead of 2.4 ms).  128 registers
+// a thread for that, with 8 bytes of spill stores.
 //
 // Reference behaviour: the reduction LAPACK's dsytrd performs inside dsyevd
 // (model/gfn2/eigensolver.cpp:1221-1254 of the reference).
