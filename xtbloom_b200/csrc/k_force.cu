@@ -49,21 +49,22 @@ __device__ __forceinline__ PairFactors pair_factors(const DevTopo& t, const doub
 // What bounds it now: 168 registers, 12 warps an SM, and the two barriers of a
 // run (512 hetero-alkanes, 2.4 ms: issue active 33 % of cycles, FP64 pipe 25 %;
 // 3.3 warps wait at a barrier per issued instruction, 2.0 for a fixed latency,
-// 1.7 for memory).  260 bytes of spill stores a thread.
+// 1.7 for memory).  256 bytes of spill stores a thread.
 // Where a run has d shells its orbital pairs are dealt to the threads in order
 // of cost: as they lie, a warp holds pairs of one and of nine Cartesian pairs
 // (400 systems of four SiCl4: GFN2 8.4 -> 5.8 ms, GFN1 16.4 -> 10.7; a thread
 // per atom pair, all alike there, 6.4 and 12.8).
 constexpr int kForceRows = 128;
 constexpr int kForceThreads = 128;
+// D: the batch has d shells (without them the kernel carries no order).
+template <bool D>
 __global__ void __launch_bounds__(kForceThreads, 3) k_force_pairs(ForceArgs f) {
   // per orbital pair: contribution to dE/dR_A and the overlap element; then
   // the shell pairs' H0 factors
   extern __shared__ double part[];
   PairFactors* pf = reinterpret_cast<PairFactors*>(part + 4 * 9 * kForceRows);
   // batches with d shells: the orbital pairs of the run in order of their cost
-  uint16_t* order = reinterpret_cast<uint16_t*>(pf + 3 * kForceRows);
-  __shared__ int cost[kCostClasses];
+  [[maybe_unused]] uint16_t* order = reinterpret_cast<uint16_t*>(pf + 3 * kForceRows);
   const DevTopo& t = f.t;
   const int s = f.list[blockIdx.y];
   const int64_t a0 = t.atom_off[s];
@@ -98,8 +99,9 @@ __global__ void __launch_bounds__(kForceThreads, 3) k_force_pairs(ForceArgs f) {
                            t.pos[3 * gA + 2] - t.pos[3 * gB + 2]};
       pf[idx] = pair_factors(t, f.cn, bs, ks, sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));
     }
-    bool sorted = false;
-    if (t.has_d) {
+    [[maybe_unused]] bool sorted = false;
+    if constexpr (D) {
+      __shared__ int cost[kCostClasses];
       auto cost_of = [&](int idx) {
         if (idx >= nrow * ncol) return -1;
         const int row = row0 + idx % nrow, col = colA + idx / nrow;
@@ -125,7 +127,8 @@ __global__ void __launch_bounds__(kForceThreads, 3) k_force_pairs(ForceArgs f) {
     }
     __syncthreads();
     for (int item = threadIdx.x; item < nrow * ncol; item += kForceThreads) {
-      const int idx = sorted ? order[item] : item;
+      int idx = item;
+      if constexpr (D) idx = sorted ? order[item] : item;
       const int row = row0 + idx % nrow, col = colA + idx / nrow;
       const int ks = t.ao_sh[o + col], bs = t.ao_sh[o + row];
       const int64_t gB = t.sh_atom[bs];
@@ -254,10 +257,15 @@ __global__ void k_force_onsite(ForceArgs f) {
 void launch_force_pairs(const ForceArgs& f, int max_atoms, cudaStream_t stream) {
   if (f.count == 0) return;
   // at most nine orbitals and three shells on an atom
-  const size_t sm = (size_t)4 * 9 * kForceRows * sizeof(double) + 3 * kForceRows * sizeof(PairFactors) +
-                    (f.t.has_d ? 9 * kForceRows * sizeof(uint16_t) : 0);
-  allow_max_dynamic_smem(k_force_pairs);
-  k_force_pairs<<<dim3(max_atoms, f.count), kForceThreads, sm, stream>>>(f);
+  const size_t sm = (size_t)4 * 9 * kForceRows * sizeof(double) + 3 * kForceRows * sizeof(PairFactors);
+  const dim3 grid(max_atoms, f.count);
+  if (f.t.has_d) {
+    allow_max_dynamic_smem(k_force_pairs<true>);
+    k_force_pairs<true><<<grid, kForceThreads, sm + 9 * kForceRows * sizeof(uint16_t), stream>>>(f);
+  } else {
+    allow_max_dynamic_smem(k_force_pairs<false>);
+    k_force_pairs<false><<<grid, kForceThreads, sm, stream>>>(f);
+  }
 }
 
 // ---------------------------------------------------------------------------
