@@ -81,7 +81,7 @@ __device__ __forceinline__ int cost_class(int lb, int mb, int lk, int mk) {
 // both table sizes.  Where an item lands within its class is not determined;
 // items must not depend on one another.  count: kCostClasses ints of shared
 // memory, zero on entry.  Call count_classes for every item (cls < 0: none),
-// by whole warps; after a barrier class_starts in one warp; after another
+// by whole warps; after a barrier class_starts in one thread; after another
 // place for every item again.
 __device__ __forceinline__ void count_classes(int cls, int* count) {
   for (int c = 0; c < kCostClasses; ++c) {
